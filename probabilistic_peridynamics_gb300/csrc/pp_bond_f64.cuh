@@ -15,6 +15,7 @@
 #pragma once
 
 #include "pp_common.cuh"
+#include "pp_exact64.cuh"
 
 namespace pp {
 
@@ -35,6 +36,75 @@ struct F64Bond {
     int nregimes;
 };
 
+// Stretch and direction cosines of one bond: s = (y - xi) / xi, q = xe / y.
+struct F64Stretch {
+    double s, qx, qy, qz;
+};
+
+// By the binary64 pipe's own operations: any inputs.
+static __device__ __noinline__ void f64_stretch_any(double x, double y, double z, double sq,
+                                                    double xi, F64Stretch* out) {
+    const double len = dsqrt(sq);
+    out->s = ddiv(dsub(len, xi), xi);
+    out->qx = ddiv(x, len);
+    out->qy = ddiv(y, len);
+    out->qz = ddiv(z, len);
+}
+
+// The same values by pp_exact64.cuh, which needs no binary64 instruction for
+// the root, the difference and the four quotients: ~140 clocks a warp and
+// slot of the integer and FP32 pipes instead of ~720 of the binary64 pipe,
+// which the other operations of the slot keep busy (fused step of the
+// 400,000-node plate, rows of 128 slots: 5.98 ms before, 3.63 ms with it; rows of
+// 32 slots 0.94 -> 0.56, of 256 slots 1.93 -> 1.06 ms).  It takes lengths within
+// 2^+-200 (squares 2^+-400) that differ by less than a factor of two, and
+// components that are zero or above 2^-700, so that no intermediate is
+// subnormal or overflows; everything else (NaN and infinities among it)
+// goes to f64_stretch_any.
+__device__ __forceinline__ F64Stretch f64_stretch(double x, double y, double z, double sq,
+                                                  double xi) {
+    using namespace exact64;
+    const uint64_t xb = double_bits(x), yb = double_bits(y), zb = double_bits(z);
+    const uint64_t sb = double_bits(sq), lb = double_bits(xi);
+    F64Stretch r;
+    uint64_t s;
+    bool ok = exponent_in(sb, 1023 - 400, 1023 + 400) && exponent_in(lb, 1023 - 200, 1023 + 200) &&
+              (lb >> 63) == 0 && zero_or_above(xb, 1023 - 700) && zero_or_above(yb, 1023 - 700) &&
+              zero_or_above(zb, 1023 - 700);
+    if (ok) {
+        const Divisor len = sqrt_rn(sb);
+        ok = relative_difference(len, divisor(lb), s);
+        r.s = bits_double(s);
+        r.qx = div_signed(xb, len);
+        r.qy = div_signed(yb, len);
+        r.qz = div_signed(zb, len);
+    }
+    if (!ok) {
+        F64Stretch t;
+        f64_stretch_any(x, y, z, sq, xi, &t);
+        r = t;
+    }
+    return r;
+}
+
+// |xi| from the squared length, correctly rounded.
+__device__ __forceinline__ double f64_length(double sq) {
+    using namespace exact64;
+    const uint64_t sb = double_bits(sq);
+    if (!exponent_in(sb, 1023 - 400, 1023 + 400) || (sb >> 63)) return dsqrt(sq);
+    const Divisor d = sqrt_rn(sb);
+    return bits_double(pack(d.m, d.e));
+}
+
+// a < b.  A binary64 comparison is an instruction of the binary64 pipe too:
+// with b positive and neither a NaN, the bits compare as signed integers.
+__device__ __forceinline__ bool f64_less(double a, double b) {
+    const int64_t ab = __double_as_longlong(a), bb = __double_as_longlong(b);
+    constexpr uint64_t kInf = 0x7FF0000000000000ull;
+    if ((uint64_t)(bb - 1) < kInf && ((uint64_t)ab << 1) <= (kInf << 1)) return ab < bb;
+    return a < b;
+}
+
 // Contribution of slot `gid` of node i.  Breaks the bond / moves its regime
 // in place exactly as the reference kernel does; counts intact bonds.
 template <bool CORR, bool TYPES>
@@ -52,13 +122,14 @@ __device__ __forceinline__ d3 f64_slot(const F64Bond& b, int64_t gid, d3 ri, d3 
     const double xe_z = dadd(dsub(uj[2], ui.z), xi_z);
     // |xi| never changes: read it when cached (the same binary64 value)
     const double xi = b.xi_len ? b.xi_len[gid]
-                               : dsqrt(dadd(dadd(dmul(xi_x, xi_x), dmul(xi_y, xi_y)),
-                                            dmul(xi_z, xi_z)));
-    const double y = dsqrt(dadd(dadd(dmul(xe_x, xe_x), dmul(xe_y, xe_y)), dmul(xe_z, xe_z)));
-    const double s = ddiv(dsub(y, xi), xi);
+                               : f64_length(dadd(dadd(dmul(xi_x, xi_x), dmul(xi_y, xi_y)),
+                                                 dmul(xi_z, xi_z)));
+    const F64Stretch st = f64_stretch(
+        xe_x, xe_y, xe_z, dadd(dadd(dmul(xe_x, xe_x), dmul(xe_y, xe_y)), dmul(xe_z, xe_z)), xi);
+    const double s = st.s;
     double f;
     if constexpr (!TYPES) {
-        if (!(s < b.s0)) {
+        if (!f64_less(s, b.s0)) {
             b.nlist[gid] = -1;
             return d3_zero();
         }
@@ -72,9 +143,9 @@ __device__ __forceinline__ d3 f64_slot(const F64Bond& b, int64_t gid, d3 ri, d3 
         // A valid bond always has 0 <= r < nregimes; clamp the table reads
         // so that a malformed regimes array cannot read out of bounds.
         const int rc = r < 0 ? 0 : (r >= nr ? nr - 1 : r);
-        if (s < b.stab[base + rc]) {
+        if (f64_less(s, b.stab[base + rc])) {
             if (r > 0 && rc > 0) {
-                if (s < b.stab[base + rc - 1]) {
+                if (f64_less(s, b.stab[base + rc - 1])) {
                     r -= 1;
                     b.regimes[gid] = r;
                 }
@@ -93,7 +164,7 @@ __device__ __forceinline__ d3 f64_slot(const F64Bond& b, int64_t gid, d3 ri, d3 
         f = dmul(f, b.vols[j]);
     }
     intact += 1;
-    return d3{dmul(f, ddiv(xe_x, y)), dmul(f, ddiv(xe_y, y)), dmul(f, ddiv(xe_z, y))};
+    return d3{dmul(f, st.qx), dmul(f, st.qy), dmul(f, st.qz)};
 }
 
 // Euler update of one DOF (peripy/cl/euler.cl:23).

@@ -46,6 +46,13 @@ __device__ __forceinline__ d3 d3_shfl_down(d3 v, int off) {
 // work-group tree order.  SL = slots per lane = max(1, L/32).  `slot(k)`
 // returns the contribution of slot k and is called exactly once for every
 // slot < L (and for no other), on all lanes together.  The sum ends in lane 0.
+//
+// A lane's slots come in bit-reversed order, so that the tree's first
+// log2(SL) steps need one pending sum per level instead of all SL values:
+// st[d] holds the finished left half of the level-d pair that the current
+// slot completes.  The loop stays rolled: one copy of the slot's code (about
+// 500 instructions), whatever SL, and log2(SL) vectors of registers (an
+// unrolled loop took 76 registers at SL = 4 and 128 with spills at SL = 32).
 template <int SL, class SlotFn>
 __device__ __forceinline__ d3 tree_reduce_f64(int lane, int L, SlotFn&& slot) {
     d3 v;
@@ -55,20 +62,26 @@ __device__ __forceinline__ d3 tree_reduce_f64(int lane, int L, SlotFn&& slot) {
             v = d3_add(v, d3_shfl_down(v, off));
         return v;
     } else {
-        constexpr int H = SL / 2;
-        d3 p[H];
+        constexpr int kLevels = SL == 2 ? 1 : SL == 4 ? 2 : SL == 8 ? 3 : SL == 16 ? 4 : 5;
+        static_assert(SL == 1 << kLevels, "SL is a power of two up to 32");
+        d3 st[kLevels];
 #pragma unroll
-        for (int k = 0; k < H; ++k) {
-            d3 a = slot(lane + 32 * k);
-            d3 b = slot(lane + 32 * (k + H));
-            p[k] = d3_add(a, b);  // tree step i = L/2
+        for (int d = 0; d < kLevels; ++d) st[d] = d3_zero();
+#pragma unroll 1
+        for (int n = 0; n < SL; ++n) {
+            v = slot(lane + 32 * static_cast<int>(__brev(n) >> (32 - kLevels)));
+            bool carry = true;
+#pragma unroll
+            for (int d = 0; d < kLevels; ++d) {
+                if (!carry) continue;
+                if ((n >> d) & 1) {
+                    v = d3_add(st[d], v);
+                } else {
+                    st[d] = v;
+                    carry = false;
+                }
+            }
         }
-#pragma unroll
-        for (int w = H / 2; w >= 1; w >>= 1) {
-#pragma unroll
-            for (int k = 0; k < w; ++k) p[k] = d3_add(p[k], p[k + w]);
-        }
-        v = p[0];
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) v = d3_add(v, d3_shfl_down(v, off));
         return v;
