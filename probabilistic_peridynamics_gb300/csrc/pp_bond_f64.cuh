@@ -54,9 +54,7 @@ static __device__ __noinline__ void f64_stretch_any(double x, double y, double z
 // The same values by pp_exact64.cuh, which needs no binary64 instruction for
 // the root, the difference and the four quotients: ~140 clocks a warp and
 // slot of the integer and FP32 pipes instead of ~720 of the binary64 pipe,
-// which the other operations of the slot keep busy (fused step of the
-// 400,000-node plate, rows of 128 slots: 5.98 ms before, 3.63 ms with it; rows of
-// 32 slots 0.94 -> 0.56, of 256 slots 1.93 -> 1.06 ms).  It takes lengths within
+// which the other operations of the slot keep busy.  It takes lengths within
 // 2^+-200 (squares 2^+-400) that differ by less than a factor of two, and
 // components that are zero or above 2^-700, so that no intermediate is
 // subnormal or overflows; everything else (NaN and infinities among it)
@@ -96,36 +94,38 @@ __device__ __forceinline__ double f64_length(double sq) {
     return bits_double(pack(d.m, d.e));
 }
 
+static __device__ __noinline__ bool f64_less_any(double a, double b) { return a < b; }
+
 // a < b.  A binary64 comparison is an instruction of the binary64 pipe too:
 // with b positive and neither a NaN, the bits compare as signed integers.
 __device__ __forceinline__ bool f64_less(double a, double b) {
     const int64_t ab = __double_as_longlong(a), bb = __double_as_longlong(b);
     constexpr uint64_t kInf = 0x7FF0000000000000ull;
     if ((uint64_t)(bb - 1) < kInf && ((uint64_t)ab << 1) <= (kInf << 1)) return ab < bb;
-    return a < b;
+    return f64_less_any(a, b);
 }
 
 // Contribution of slot `gid` of node i.  Breaks the bond / moves its regime
 // in place exactly as the reference kernel does; counts intact bonds.
 template <bool CORR, bool TYPES>
-__device__ __forceinline__ d3 f64_slot(const F64Bond& b, int64_t gid, d3 ri, d3 ui,
+__device__ __forceinline__ d3 f64_slot(const F64Ops& op, const F64Bond& b, int64_t gid, d3 ri, d3 ui,
                                        int& intact) {
     const int j = b.nlist[gid];
     if (j == -1) return d3_zero();
     const double* rj = b.r0 + 3 * (int64_t)j;
     const double* uj = b.u + 3 * (int64_t)j;
-    const double xi_x = dsub(rj[0], ri.x);
-    const double xi_y = dsub(rj[1], ri.y);
-    const double xi_z = dsub(rj[2], ri.z);
-    const double xe_x = dadd(dsub(uj[0], ui.x), xi_x);
-    const double xe_y = dadd(dsub(uj[1], ui.y), xi_y);
-    const double xe_z = dadd(dsub(uj[2], ui.z), xi_z);
+    const double xi_x = op.sub(rj[0], ri.x);
+    const double xi_y = op.sub(rj[1], ri.y);
+    const double xi_z = op.sub(rj[2], ri.z);
+    const double xe_x = op.add(op.sub(uj[0], ui.x), xi_x);
+    const double xe_y = op.add(op.sub(uj[1], ui.y), xi_y);
+    const double xe_z = op.add(op.sub(uj[2], ui.z), xi_z);
     // |xi| never changes: read it when cached (the same binary64 value)
     const double xi = b.xi_len ? b.xi_len[gid]
-                               : f64_length(dadd(dadd(dmul(xi_x, xi_x), dmul(xi_y, xi_y)),
-                                                 dmul(xi_z, xi_z)));
+                               : f64_length(op.add(op.add(op.mul(xi_x, xi_x), op.mul(xi_y, xi_y)),
+                                                 op.mul(xi_z, xi_z)));
     const F64Stretch st = f64_stretch(
-        xe_x, xe_y, xe_z, dadd(dadd(dmul(xe_x, xe_x), dmul(xe_y, xe_y)), dmul(xe_z, xe_z)), xi);
+        xe_x, xe_y, xe_z, op.add(op.add(op.mul(xe_x, xe_x), op.mul(xe_y, xe_y)), op.mul(xe_z, xe_z)), xi);
     const double s = st.s;
     double f;
     if constexpr (!TYPES) {
@@ -133,9 +133,9 @@ __device__ __forceinline__ d3 f64_slot(const F64Bond& b, int64_t gid, d3 ri, d3 
             b.nlist[gid] = -1;
             return d3_zero();
         }
-        f = dmul(s, b.k);
-        if constexpr (CORR) f = dmul(f, b.sc[gid]);
-        f = dmul(f, b.vols[j]);
+        f = op.mul(s, b.k);
+        if constexpr (CORR) f = op.mul(f, b.sc[gid]);
+        f = op.mul(f, b.vols[j]);
     } else {
         const int nr = b.nregimes;
         const int base = b.btypes[gid] * nr;
@@ -159,12 +159,12 @@ __device__ __forceinline__ d3 f64_slot(const F64Bond& b, int64_t gid, d3 ri, d3 
             return d3_zero();
         }
         const int rr = r < 0 ? 0 : r;
-        f = dadd(dmul(s, b.ktab[base + rr]), b.ctab[base + rr]);
-        if constexpr (CORR) f = dmul(f, b.sc[gid]);
-        f = dmul(f, b.vols[j]);
+        f = op.add(op.mul(s, b.ktab[base + rr]), b.ctab[base + rr]);
+        if constexpr (CORR) f = op.mul(f, b.sc[gid]);
+        f = op.mul(f, b.vols[j]);
     }
     intact += 1;
-    return d3{dmul(f, st.qx), dmul(f, st.qy), dmul(f, st.qz)};
+    return d3{op.mul(f, st.qx), op.mul(f, st.qy), op.mul(f, st.qz)};
 }
 
 // Euler update of one DOF (peripy/cl/euler.cl:23).
@@ -189,7 +189,7 @@ __device__ __forceinline__ double velocity_verlet_u(double u, double& ud, double
                                                     double f, int bct, double bcv,
                                                     double rho, double bc_scale,
                                                     double damping, double dt) {
-    const double half = ddiv(dt, 2.0);
+    const double half = dmul(dt, 0.5);  // dt / 2
     const double ud1 = dadd(ud, dmul(half, udd));
     const double udd1 = ddiv(dsub(f, dmul(damping, ud1)), rho);
     ud = dadd(ud1, dmul(half, udd1));

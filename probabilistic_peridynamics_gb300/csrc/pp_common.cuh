@@ -42,50 +42,97 @@ __device__ __forceinline__ d3 d3_shfl_down(d3 v, int off) {
               __shfl_down_sync(kFull, v.z, off)};
 }
 
+// Additions and products as fused multiply-adds: a + b = fma(a, 1, b) and
+// a b = fma(a, b, -0) are the same correctly rounded values (signed zeros
+// included).  On GB300 a DFMA whose three operands are registers issues every
+// 17 clocks per warp and SM, a DADD or DMUL every 20 (measured 1.89 against
+// 1.59 lanes/clk/SM), so the constants are kept in registers that the
+// compiler cannot see through.
+struct F64Ops {
+    double one, nzero;
+    // `word`: a shared word of the block, written before a barrier
+    __device__ __forceinline__ explicit F64Ops(const volatile double* word) {
+        one = *word;
+        nzero = __longlong_as_double(__double_as_longlong(one) ^ 0xBFF0000000000000ll);
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(-b, one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nzero); }
+};
+
+__device__ __forceinline__ double shfl_xor(double v, int off) {
+    return __shfl_xor_sync(kFull, v, off);
+}
+
+// Levels of pending sums that tree_reduce_f64 keeps per thread.
+template <int SL>
+struct TreeLevels {
+    static constexpr int value = 1 + TreeLevels<SL / 2>::value;
+};
+template <>
+struct TreeLevels<1> {
+    static constexpr int value = 0;
+};
+
+// Bytes of tree_reduce_f64's stack for a block.
+template <int SL>
+constexpr size_t tree_stack_bytes(int threads) {
+    return sizeof(double) * 3 * TreeLevels<SL>::value * threads;
+}
+
 // Reduce per-slot binary64 vectors of one node held by one warp, in the
 // work-group tree order.  SL = slots per lane = max(1, L/32).  `slot(k)`
 // returns the contribution of slot k and is called exactly once for every
-// slot < L (and for no other), on all lanes together.  The sum ends in lane 0.
+// slot < L (and for no other), on all lanes together.  Returns the sum's x on
+// lane 0, z on lane 8 and y on lane 16.
 //
 // A lane's slots come in bit-reversed order, so that the tree's first
-// log2(SL) steps need one pending sum per level instead of all SL values:
-// st[d] holds the finished left half of the level-d pair that the current
-// slot completes.  The loop stays rolled: one copy of the slot's code (about
-// 500 instructions), whatever SL, and log2(SL) vectors of registers (an
-// unrolled loop took 76 registers at SL = 4 and 128 with spills at SL = 32).
+// log2(SL) steps need one pending sum per level: `stack` (shared memory, 3
+// log2(SL) words per thread, `stride` threads) holds the finished left half
+// of the pair that a later slot completes.  The loop stays rolled (one copy
+// of the slot's code, whatever SL), and the additions are branched around,
+// not predicated: a predicated DADD still takes the binary64 pipe's time.
+//
+// The last five steps pack the components: a step's lower half computes one
+// component while the upper half computes another (addition commutes, so the
+// sums are the tree's own): 6 additions a warp instead of 15.
 template <int SL, class SlotFn>
-__device__ __forceinline__ d3 tree_reduce_f64(int lane, int L, SlotFn&& slot) {
+__device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, int L, double* stack,
+                                                  int stride, SlotFn&& slot) {
     d3 v;
     if constexpr (SL == 1) {
         v = (lane < L) ? slot(lane) : d3_zero();
-        for (int off = (L >> 1) < 16 ? (L >> 1) : 16; off >= 1; off >>= 1)
-            v = d3_add(v, d3_shfl_down(v, off));
-        return v;
+        if (L < 32) {
+            for (int off = L >> 1; off >= 1; off >>= 1) v = d3_add(v, d3_shfl_down(v, off));
+            const double y = __shfl_sync(kFull, v.y, 0), z = __shfl_sync(kFull, v.z, 0);
+            return lane == 0 ? v.x : (lane == 8 ? z : y);
+        }
     } else {
-        constexpr int kLevels = SL == 2 ? 1 : SL == 4 ? 2 : SL == 8 ? 3 : SL == 16 ? 4 : 5;
-        static_assert(SL == 1 << kLevels, "SL is a power of two up to 32");
-        d3 st[kLevels];
-#pragma unroll
-        for (int d = 0; d < kLevels; ++d) st[d] = d3_zero();
 #pragma unroll 1
         for (int n = 0; n < SL; ++n) {
-            v = slot(lane + 32 * static_cast<int>(__brev(n) >> (32 - kLevels)));
-            bool carry = true;
-#pragma unroll
-            for (int d = 0; d < kLevels; ++d) {
-                if (!carry) continue;
-                if ((n >> d) & 1) {
-                    v = d3_add(st[d], v);
-                } else {
-                    st[d] = v;
-                    carry = false;
-                }
+            v = slot(lane + 32 * static_cast<int>(__brev(n) >> (32 - TreeLevels<SL>::value)));
+            double* p = stack;
+            int m = n;
+#pragma unroll 1
+            while (m & 1) {
+                v = d3{op.add(p[0], v.x), op.add(p[stride], v.y), op.add(p[2 * stride], v.z)};
+                p += 3 * stride;
+                m >>= 1;
+            }
+            if (n != SL - 1) {
+                p[0] = v.x;
+                p[stride] = v.y;
+                p[2 * stride] = v.z;
             }
         }
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) v = d3_add(v, d3_shfl_down(v, off));
-        return v;
     }
+    const bool up16 = lane & 16, up8 = lane & 8;
+    const double xy = op.add(up16 ? v.y : v.x, shfl_xor(up16 ? v.x : v.y, 16));
+    const double z = op.add(v.z, shfl_xor(v.z, 16));
+    double t = op.add(up8 ? z : xy, shfl_xor(up8 ? xy : z, 8));
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1) t = op.add(t, shfl_xor(t, off));
+    return t;
 }
 
 // ------------------------------------------------------------ double-float

@@ -19,15 +19,23 @@
 namespace pp {
 namespace {
 
-constexpr int kDefaultWarps = 8;
+// Four warps a block: 24 warps per SM at 80 registers, and a block's node
+// updates wait for four warps only (400,000-node plate, rows of 128 slots:
+// 2.69 ms against 2.72 with eight; 2000 nodes 19.8 against 20.6 us).
+constexpr int kDefaultWarps = 4;
 
 // One warp per node for the bond phase; the node updates of the block's
 // nodes then run one thread per DOF (the update's binary64 instructions
 // would otherwise occupy GB300's FP64 pipe for a whole warp per 3 lanes).
 template <int SL, bool CORR, bool TYPES>
-__global__ void __launch_bounds__(256) k_fused_f64(pp_fused_args a, int parity, Launch l) {
-    __shared__ double s_f[32][3];
-    __shared__ int s_cnt[32];
+__global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parity, Launch l) {
+    __shared__ double s_f[8][3];
+    __shared__ int s_cnt[8];
+    __shared__ double s_one;
+    extern __shared__ double s_stack[];
+    if (threadIdx.x == 0) s_one = 1.0;
+    __syncthreads();
+    const F64Ops op(&s_one);
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5;
@@ -55,16 +63,17 @@ __global__ void __launch_bounds__(256) k_fused_f64(pp_fused_args a, int parity, 
         const d3 ui{u[o3], u[o3 + 1], u[o3 + 2]};
         const int64_t row = (int64_t)i * a.max_neigh;
         int intact = 0;
-        const d3 f = tree_reduce_f64<SL>(lane, a.max_neigh, [&](int k) {
-            return f64_slot<CORR, TYPES>(b, row + k, ri, ui, intact);
+        const double f = tree_reduce_f64<SL>(op, lane, a.max_neigh, s_stack + threadIdx.x,
+                                             blockDim.x, [&](int k) {
+            return f64_slot<CORR, TYPES>(op, b, row + k, ri, ui, intact);
         });
         const int count = __reduce_add_sync(kFull, intact);
         if (lane == 0) {
-            s_f[warp][0] = f.x;
-            s_f[warp][1] = f.y;
-            s_f[warp][2] = f.z;
+            s_f[warp][0] = f;
             s_cnt[warp] = count;
         }
+        if (lane == 16) s_f[warp][1] = f;
+        if (lane == 8) s_f[warp][2] = f;
     }
     __syncthreads();
     const int t = threadIdx.x;
@@ -164,7 +173,8 @@ template <int SL, bool CORR, bool TYPES>
 void launch_f64_variant(const pp_fused_args& a, int parity, const Launch& l, cudaStream_t st) {
     const int wpb = a.nodes_per_block > 0 ? a.nodes_per_block : kDefaultWarps;
     const dim3 grid((a.nnodes + wpb - 1) / wpb), block(32 * wpb);
-    k_fused_f64<SL, CORR, TYPES><<<grid, block, 0, st>>>(a, parity, l);
+    k_fused_f64<SL, CORR, TYPES>
+        <<<grid, block, tree_stack_bytes<SL>(32 * wpb), st>>>(a, parity, l);
 }
 
 template <int SL>

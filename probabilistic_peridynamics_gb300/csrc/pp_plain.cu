@@ -11,11 +11,16 @@
 namespace pp {
 namespace {
 
-constexpr int kWarpsPerBlock = 8;
+constexpr int kWarpsPerBlock = 4;
 
 template <int SL, bool CORR, bool TYPES>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_bond_force(pp_bond_force_args a) {
+    __shared__ double s_one;
+    extern __shared__ double s_stack[];
+    if (threadIdx.x == 0) s_one = 1.0;
+    __syncthreads();
+    const F64Ops op(&s_one);
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (i >= a.nnodes) return;  // warp-uniform
@@ -37,17 +42,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     const d3 ui{a.u[3 * (int64_t)i], a.u[3 * (int64_t)i + 1], a.u[3 * (int64_t)i + 2]};
     const int64_t row = (int64_t)i * a.max_neigh;
     int intact = 0;
-    const d3 f = tree_reduce_f64<SL>(lane, a.max_neigh, [&](int k) {
-        return f64_slot<CORR, TYPES>(b, row + k, ri, ui, intact);
-    });
-    if (lane == 0) {
-        const int64_t o = 3 * (int64_t)i;
-        a.body_force[o] = f.x;
-        a.body_force[o + 1] = f.y;
-        a.body_force[o + 2] = f.z;
-        a.force[o] = force_with_bc(f.x, a.fc_types[o], a.fc_values[o], a.fc_scale);
-        a.force[o + 1] = force_with_bc(f.y, a.fc_types[o + 1], a.fc_values[o + 1], a.fc_scale);
-        a.force[o + 2] = force_with_bc(f.z, a.fc_types[o + 2], a.fc_values[o + 2], a.fc_scale);
+    const double f = tree_reduce_f64<SL>(
+        op, lane, a.max_neigh, s_stack + threadIdx.x, kWarpsPerBlock * 32,
+        [&](int k) { return f64_slot<CORR, TYPES>(op, b, row + k, ri, ui, intact); });
+    if (lane == 0 || lane == 8 || lane == 16) {  // x, z, y
+        const int64_t o = 3 * (int64_t)i + (lane == 0 ? 0 : (lane == 8 ? 2 : 1));
+        a.body_force[o] = f;
+        a.force[o] = force_with_bc(f, a.fc_types[o], a.fc_values[o], a.fc_scale);
     }
 }
 
@@ -57,10 +58,11 @@ int launch_bond_force(const pp_bond_force_args& a, cudaStream_t st) {
     const dim3 block(kWarpsPerBlock * 32);
     const bool corr = a.stiffness_corrections != nullptr;
     const bool types = a.bond_types != nullptr;
-    if (!corr && !types) k_bond_force<SL, false, false><<<grid, block, 0, st>>>(a);
-    if (corr && !types) k_bond_force<SL, true, false><<<grid, block, 0, st>>>(a);
-    if (!corr && types) k_bond_force<SL, false, true><<<grid, block, 0, st>>>(a);
-    if (corr && types) k_bond_force<SL, true, true><<<grid, block, 0, st>>>(a);
+    constexpr size_t dyn = tree_stack_bytes<SL>(kWarpsPerBlock * 32);
+    if (!corr && !types) k_bond_force<SL, false, false><<<grid, block, dyn, st>>>(a);
+    if (corr && !types) k_bond_force<SL, true, false><<<grid, block, dyn, st>>>(a);
+    if (!corr && types) k_bond_force<SL, false, true><<<grid, block, dyn, st>>>(a);
+    if (corr && types) k_bond_force<SL, true, true><<<grid, block, dyn, st>>>(a);
     return launch_status();
 }
 
