@@ -16,6 +16,7 @@
 
 #include "pp_common.cuh"
 #include "pp_exact64.cuh"
+#include "pp_fused.cuh"
 
 namespace pp {
 
@@ -37,18 +38,21 @@ struct F64Bond {
 };
 
 // Stretch and direction cosines of one bond: s = (y - xi) / xi, q = xe / y.
+// Kept as bits: where two paths join, the compiler merges doubles with an
+// instruction of the binary64 pipe each.
 struct F64Stretch {
-    double s, qx, qy, qz;
+    uint64_t s, qx, qy, qz;
 };
 
 // By the binary64 pipe's own operations: any inputs.
 static __device__ __noinline__ void f64_stretch_any(double x, double y, double z, double sq,
                                                     double xi, F64Stretch* out) {
+    using exact64::double_bits;
     const double len = dsqrt(sq);
-    out->s = ddiv(dsub(len, xi), xi);
-    out->qx = ddiv(x, len);
-    out->qy = ddiv(y, len);
-    out->qz = ddiv(z, len);
+    out->s = double_bits(ddiv(dsub(len, xi), xi));
+    out->qx = double_bits(ddiv(x, len));
+    out->qy = double_bits(ddiv(y, len));
+    out->qz = double_bits(ddiv(z, len));
 }
 
 // The same values by pp_exact64.cuh, which needs no binary64 instruction for
@@ -64,18 +68,16 @@ __device__ __forceinline__ F64Stretch f64_stretch(double x, double y, double z, 
     using namespace exact64;
     const uint64_t xb = double_bits(x), yb = double_bits(y), zb = double_bits(z);
     const uint64_t sb = double_bits(sq), lb = double_bits(xi);
-    F64Stretch r;
-    uint64_t s;
-    bool ok = exponent_in(sb, 1023 - 400, 1023 + 400) && exponent_in(lb, 1023 - 200, 1023 + 200) &&
-              (lb >> 63) == 0 && zero_or_above(xb, 1023 - 700) && zero_or_above(yb, 1023 - 700) &&
+    F64Stretch r{0, 0, 0, 0};
+    bool ok = positive_in(sb, 1023 - 400, 1023 + 400) && positive_in(lb, 1023 - 200, 1023 + 200) &&
+              zero_or_above(xb, 1023 - 700) && zero_or_above(yb, 1023 - 700) &&
               zero_or_above(zb, 1023 - 700);
     if (ok) {
         const Divisor len = sqrt_rn(sb);
-        ok = relative_difference(len, divisor(lb), s);
-        r.s = bits_double(s);
-        r.qx = div_signed(xb, len);
-        r.qy = div_signed(yb, len);
-        r.qz = div_signed(zb, len);
+        ok = relative_difference(len, divisor(lb), r.s);
+        r.qx = div_bits(xb, len);
+        r.qy = div_bits(yb, len);
+        r.qz = div_bits(zb, len);
     }
     if (!ok) {
         F64Stretch t;
@@ -89,7 +91,7 @@ __device__ __forceinline__ F64Stretch f64_stretch(double x, double y, double z, 
 __device__ __forceinline__ double f64_length(double sq) {
     using namespace exact64;
     const uint64_t sb = double_bits(sq);
-    if (!exponent_in(sb, 1023 - 400, 1023 + 400) || (sb >> 63)) return dsqrt(sq);
+    if (!positive_in(sb, 1023 - 400, 1023 + 400)) return dsqrt(sq);
     const Divisor d = sqrt_rn(sb);
     return bits_double(pack(d.m, d.e));
 }
@@ -105,37 +107,18 @@ __device__ __forceinline__ bool f64_less(double a, double b) {
     return f64_less_any(a, b);
 }
 
-// Contribution of slot `gid` of node i.  Breaks the bond / moves its regime
-// in place exactly as the reference kernel does; counts intact bonds.
+// The damage law of the bond in slot `gid` at stretch s, towards a neighbour
+// of volume vol: breaks the bond / moves its regime in place exactly as the
+// reference kernel does.  True when the bond stays; f is then its force.
 template <bool CORR, bool TYPES>
-__device__ __forceinline__ d3 f64_slot(const F64Ops& op, const F64Bond& b, int64_t gid, d3 ri, d3 ui,
-                                       int& intact) {
-    const int j = b.nlist[gid];
-    if (j == -1) return d3_zero();
-    const double* rj = b.r0 + 3 * (int64_t)j;
-    const double* uj = b.u + 3 * (int64_t)j;
-    const double xi_x = op.sub(rj[0], ri.x);
-    const double xi_y = op.sub(rj[1], ri.y);
-    const double xi_z = op.sub(rj[2], ri.z);
-    const double xe_x = op.add(op.sub(uj[0], ui.x), xi_x);
-    const double xe_y = op.add(op.sub(uj[1], ui.y), xi_y);
-    const double xe_z = op.add(op.sub(uj[2], ui.z), xi_z);
-    // |xi| never changes: read it when cached (the same binary64 value)
-    const double xi = b.xi_len ? b.xi_len[gid]
-                               : f64_length(op.add(op.add(op.mul(xi_x, xi_x), op.mul(xi_y, xi_y)),
-                                                 op.mul(xi_z, xi_z)));
-    const F64Stretch st = f64_stretch(
-        xe_x, xe_y, xe_z, op.add(op.add(op.mul(xe_x, xe_x), op.mul(xe_y, xe_y)), op.mul(xe_z, xe_z)), xi);
-    const double s = st.s;
-    double f;
+__device__ __forceinline__ bool f64_bond_law(const F64Ops& op, const F64Bond& b, int64_t gid,
+                                             double s, double vol, double& f) {
     if constexpr (!TYPES) {
         if (!f64_less(s, b.s0)) {
             b.nlist[gid] = -1;
-            return d3_zero();
+            return false;
         }
         f = op.mul(s, b.k);
-        if constexpr (CORR) f = op.mul(f, b.sc[gid]);
-        f = op.mul(f, b.vols[j]);
     } else {
         const int nr = b.nregimes;
         const int base = b.btypes[gid] * nr;
@@ -156,15 +139,65 @@ __device__ __forceinline__ d3 f64_slot(const F64Ops& op, const F64Bond& b, int64
         }
         if (r >= nr) {
             b.nlist[gid] = -1;
-            return d3_zero();
+            return false;
         }
         const int rr = r < 0 ? 0 : r;
         f = op.add(op.mul(s, b.ktab[base + rr]), b.ctab[base + rr]);
-        if constexpr (CORR) f = op.mul(f, b.sc[gid]);
-        f = op.mul(f, b.vols[j]);
     }
+    if constexpr (CORR) f = op.mul(f, b.sc[gid]);
+    f = op.mul(f, vol);
+    return true;
+}
+
+// Deformed bond vector from node i (r0 ri, displacement ui) to node j, and
+// the reference vector.
+__device__ __forceinline__ d3 f64_bond_vector(const F64Ops& op, const F64Bond& b, int j, d3 ri,
+                                              d3 ui, d3& xi) {
+    const double* rj = b.r0 + 3 * (int64_t)j;
+    const double* uj = b.u + 3 * (int64_t)j;
+    xi = d3{op.sub(rj[0], ri.x), op.sub(rj[1], ri.y), op.sub(rj[2], ri.z)};
+    return d3{op.add(op.sub(uj[0], ui.x), xi.x), op.add(op.sub(uj[1], ui.y), xi.y),
+              op.add(op.sub(uj[2], ui.z), xi.z)};
+}
+
+__device__ __forceinline__ double f64_square(const F64Ops& op, const d3& v) {
+    return op.add(op.add(op.mul(v.x, v.x), op.mul(v.y, v.y)), op.mul(v.z, v.z));
+}
+
+__device__ __forceinline__ d3 f64_force(const F64Ops& op, double f, const F64Stretch& st) {
+    return d3{op.mul(f, __longlong_as_double(st.qx)), op.mul(f, __longlong_as_double(st.qy)),
+              op.mul(f, __longlong_as_double(st.qz))};
+}
+
+// Contribution of slot `gid` of node i; counts intact bonds.
+template <bool CORR, bool TYPES>
+__device__ __forceinline__ d3 f64_slot(const F64Ops& op, const F64Bond& b, int64_t gid, d3 ri,
+                                       d3 ui, int& intact) {
+    const int j = b.nlist[gid];
+    if (j == -1) return d3_zero();
+    d3 xi;
+    const d3 xe = f64_bond_vector(op, b, j, ri, ui, xi);
+    // |xi| never changes: read it when cached (the same binary64 value)
+    const double len = b.xi_len ? b.xi_len[gid] : f64_length(f64_square(op, xi));
+    const F64Stretch st = f64_stretch(xe.x, xe.y, xe.z, f64_square(op, xe), len);
+    double f;
+    if (!f64_bond_law<CORR, TYPES>(op, b, gid, __longlong_as_double(st.s), b.vols[j], f))
+        return d3_zero();
     intact += 1;
-    return d3{op.mul(f, st.qx), op.mul(f, st.qy), op.mul(f, st.qz)};
+    return f64_force(op, f, st);
+}
+
+static __device__ __noinline__ double f64_divide_any(double a, double b) { return ddiv(a, b); }
+
+// a / b: on the integer pipe where a and b are within 2^+-400 (a may be
+// zero) and b is positive, as densities are; else the binary64 pipe's own.
+__device__ __forceinline__ double f64_divide(double a, double b) {
+    using namespace exact64;
+    const uint64_t ab = double_bits(a), bb = double_bits(b);
+    const bool ok = positive_in(bb, 1023 - 400, 1023 + 400) &&
+                    (is_zero(ab) || positive_in(ab & 0x7FFFFFFFFFFFFFFFull, 1023 - 400, 1023 + 400));
+    if (!ok) return f64_divide_any(a, b);
+    return div_signed(ab, divisor(bb));
 }
 
 // Euler update of one DOF (peripy/cl/euler.cl:23).
@@ -178,7 +211,7 @@ __device__ __forceinline__ double euler_cromer_u(double u, double& ud, double& u
                                                  int bct, double bcv, double rho,
                                                  double bc_scale, double damping,
                                                  double dt) {
-    const double uddi = ddiv(dsub(f, dmul(damping, ud)), rho);
+    const double uddi = f64_divide(dsub(f, dmul(damping, ud)), rho);
     udd = uddi;
     ud = dadd(ud, dmul(uddi, dt));
     return bct == 0 ? dadd(u, dmul(dt, ud)) : dmul(bc_scale, bcv);
@@ -191,7 +224,7 @@ __device__ __forceinline__ double velocity_verlet_u(double u, double& ud, double
                                                     double damping, double dt) {
     const double half = dmul(dt, 0.5);  // dt / 2
     const double ud1 = dadd(ud, dmul(half, udd));
-    const double udd1 = ddiv(dsub(f, dmul(damping, ud1)), rho);
+    const double udd1 = f64_divide(dsub(f, dmul(damping, ud1)), rho);
     ud = dadd(ud1, dmul(half, udd1));
     udd = udd1;
     return bct == 0 ? dadd(u, dmul(dt, dadd(ud, dmul(half, udd1)))) : dmul(bc_scale, bcv);
@@ -203,9 +236,61 @@ __device__ __forceinline__ double force_with_bc(double body, int fct, double fcv
     return fct == 0 ? body : dadd(body, dmul(fc_scale, fcv));
 }
 
-// Damage of one node (peridynamics.cl:606-608).
+// Damage of one node (peridynamics.cl:606-608): 1 - intact / family.  The
+// integers become significands directly (a conversion is an instruction of
+// the binary64 pipe).
 __device__ __forceinline__ double damage_of(int intact, int family) {
-    return dsub(1.0, ddiv((double)intact, (double)family));
+    using namespace exact64;
+    if (family <= 0 || intact < 0) return dsub(1.0, ddiv((double)intact, (double)family));
+    if (intact == 0) return 1.0;
+    return dsub(1.0, div_signed(int_bits(intact), divisor(int_bits(family))));
+}
+
+// Node updates of a block's `wpb` nodes from their bond forces (s_f) and
+// intact counts: one thread per DOF, then one per node for the damage (a
+// warp-wide update of one node's three DOFs would hold the binary64 pipe as
+// long).
+__device__ __forceinline__ void f64_node_phase(const pp_fused_args& a, int parity,
+                                               const StepMags& m, int node0, int wpb,
+                                               const double (*s_f)[3], const int* s_cnt) {
+    const double* __restrict__ u = a.u[parity];
+    const int t = threadIdx.x;
+    if (t < 3 * wpb) {
+        const int li = t / 3, d = t % 3;
+        const int n = node0 + li;
+        if (n < a.nnodes) {
+            const int64_t o = 3 * (int64_t)n + d;
+            const double body = s_f[li][d];
+            a.body_force[o] = body;
+            const double frc = force_with_bc(body, a.fc_types[o], a.fc_values[o], m.force);
+            a.force[o] = frc;
+            const int bct = a.bc_types[o];
+            const double bcv = a.bc_values[o];
+            double unew;
+            if (a.integrator == PP_EULER) {
+                unew = euler_u(u[o], frc, bct, bcv, m.disp, a.dt);
+            } else {
+                double v = a.ud[o];
+                double acc = a.udd[o];
+                if (a.integrator == PP_EULER_CROMER)
+                    unew = euler_cromer_u(u[o], v, acc, frc, bct, bcv, a.densities[o], m.disp,
+                                          a.damping, a.dt);
+                else
+                    unew = velocity_verlet_u(u[o], v, acc, frc, bct, bcv, a.densities[o],
+                                             m.disp, a.damping, a.dt);
+                a.ud[o] = v;
+                a.udd[o] = acc;
+            }
+            a.u[parity ^ 1][o] = unew;
+        }
+    } else if (t < 4 * wpb) {
+        const int n = node0 + (t - 3 * wpb);
+        if (n < a.nnodes) {
+            const int count = s_cnt[t - 3 * wpb];
+            a.n_neigh[n] = count;
+            a.damage[n] = damage_of(count, a.family[n]);
+        }
+    }
 }
 
 }  // namespace pp

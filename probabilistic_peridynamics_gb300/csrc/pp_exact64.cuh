@@ -125,6 +125,10 @@ PP_HD float fma32(float a, float b, float c) {
 constexpr float kMagic = 12582912.0f;
 constexpr uint32_t kMagicBits = 0x4B400000u;
 PP_HD int32_t magic_int(float m) { return (int32_t)(float_bits(m) - kMagicBits); }
+// float(v) for |v| < 2^22, exactly.  (An integer-to-float conversion runs on
+// GB300's binary64 pipe, 16 clocks a warp: four of them took a seventh of the
+// fused step.)
+PP_HD float small_float(int32_t v) { return bits_float(kMagicBits + (uint32_t)v) - kMagic; }
 
 // The low 32 bits of v >> s (0 < s < 32).
 PP_HD uint32_t shift_word(uint64_t v, int s) {
@@ -169,7 +173,7 @@ PP_HD uint32_t reciprocal_word(uint64_t m, float r) {
     const uint32_t t = shift_word(m, 21);
     const uint64_t prod = (uint64_t)v0 * t;
     const int32_t n = (int32_t)shift_word(prod, 20);  // (prod - 2^63) >> 20
-    const float c = fma32((float)n, r * -0x1p-11f, kMagic);
+    const float c = fma32(small_float(n), r * -0x1p-11f, kMagic);
     return v0 + (uint32_t)magic_int(c) - 3u;
 }
 
@@ -186,17 +190,18 @@ PP_HD Divisor sqrt_rn(uint64_t bits) {
     g = g > 1.0f ? g : 1.0f;
     g = g < 1.99999988f ? g : 1.99999988f;
     const uint32_t yh = float_bits(g) - 0x3F000000u;
-    // first residual mm - (8 yh)^2, |.| < 2^33.2; correction in 2^10 ulp
+    // first residual mm - (8 yh)^2, |.| < 2^33.2; correction in 2^10 ulp, 3.2
+    // of which are its error (2 from the dropped bits of the residual)
     const uint32_t y8 = yh << 3;
     const uint64_t r1 = mm - (uint64_t)y8 * y8;
-    const int32_t p1 = (int32_t)shift_word(r1, 3);
-    const int32_t t1 = magic_int(fma32((float)p1, r * 0x1p-8f, kMagic));
+    const int32_t p1 = (int32_t)shift_word(r1, 12);
+    const int32_t t1 = magic_int(fma32(small_float(p1), r * 2.0f, kMagic));
     const uint64_t z = ((uint64_t)yh << 19) + (uint64_t)(int64_t)t1;
-    // second residual mm 2^32 - z^2, |.| < 2^45; correction in ulp,
-    // then |Y - sqrt| < 0.5 + 2^-10
+    // second residual mm 2^32 - z^2, |.| < 2^45.8; correction in ulp, then
+    // |Y - sqrt| < 0.5 + 2^-8
     const uint64_t r2 = (mm << 32) - z * z;
-    const int32_t p2 = (int32_t)shift_word(r2, 16);
-    const int32_t t2 = magic_int(fma32((float)p2, r * 0x1p-17f, kMagic));
+    const int32_t p2 = (int32_t)shift_word(r2, 24);
+    const int32_t t2 = magic_int(fma32(small_float(p2), r * 0x1p-9f, kMagic));
     uint64_t y = (z << 10) + (uint64_t)(int64_t)t2;
     // exact rounding: r3 = mm 2^52 - Y^2 must lie in (-Y, Y]
     const int64_t r3 = (int64_t)((mm << 52) - y * y);
@@ -230,14 +235,26 @@ PP_HD Num div_rn(const Num& a, const Divisor& d) {
     return Num{q, a.e - d.e + 1023 - (int32_t)lt};
 }
 
+// +0 or -0, from the two words: the compiler turns a test of the whole into
+// a comparison on the binary64 pipe.
+PP_HD bool is_zero(uint64_t bits) {
+    uint32_t hi = (uint32_t)(bits >> 32) << 1, lo = (uint32_t)bits;
+#ifdef __CUDA_ARCH__
+    asm("" : "+r"(hi), "+r"(lo));
+#endif
+    return (hi | lo) == 0;
+}
+
 // a / d for a of either sign, zero included.  Neither NaN nor infinite; a
 // nonzero a is normal, and so is the quotient (the caller checks).
-PP_HD double div_signed(uint64_t a, const Divisor& d) {
+PP_HD uint64_t div_bits(uint64_t a, const Divisor& d) {
     const Num q = div_rn(unpack(a), d);
     const uint64_t sign = a & 0x8000000000000000ull;
     const uint64_t bits = sign | pack(q.m, q.e);
-    return bits_double((a << 1) == 0 ? a : bits);
+    return is_zero(a) ? a : bits;
 }
+
+PP_HD double div_signed(uint64_t a, const Divisor& d) { return bits_double(div_bits(a, d)); }
 
 PP_HD int leading_zeros(uint64_t v) {
 #ifdef __CUDA_ARCH__
@@ -246,6 +263,12 @@ PP_HD int leading_zeros(uint64_t v) {
 #else
     return v ? __builtin_clzll(v) : 64;
 #endif
+}
+
+// bits of a positive integer as a binary64 number.
+PP_HD uint64_t int_bits(int v) {
+    const int up = leading_zeros((uint64_t)(uint32_t)v) - 11;
+    return ((uint64_t)(uint32_t)v << up) + ((uint64_t)(1023 + 51 - up) << 52);
 }
 
 // bits of (y - x) / x, both positive and normal.  False when the exponents
@@ -263,13 +286,12 @@ PP_HD bool relative_difference(const Divisor& y, const Divisor& x, uint64_t& bit
 
 // Zero, or a number whose exponent field is at least lo.
 PP_HD bool zero_or_above(uint64_t bits, uint32_t lo) {
-    return ((uint32_t)(bits >> 52) & 0x7FFu) >= lo || (bits << 1) == 0;
+    return ((uint32_t)(bits >> 32) << 1) >= (lo << 21) || is_zero(bits);
 }
 
-// Is `bits` a normal number of exponent field lo .. hi?
-PP_HD bool exponent_in(uint64_t bits, uint32_t lo, uint32_t hi) {
-    const uint32_t e = ((uint32_t)(bits >> 52)) & 0x7FFu;
-    return e - lo <= hi - lo;
+// Is `bits` a positive number of exponent field lo .. hi (0 < lo)?
+PP_HD bool positive_in(uint64_t bits, uint32_t lo, uint32_t hi) {
+    return (uint32_t)(bits >> 52) - lo <= hi - lo;
 }
 
 }  // namespace exact64

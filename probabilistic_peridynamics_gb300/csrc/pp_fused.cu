@@ -76,43 +76,7 @@ __global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parit
         if (lane == 8) s_f[warp][2] = f;
     }
     __syncthreads();
-    const int t = threadIdx.x;
-    if (t < 3 * wpb) {
-        const int li = t / 3, d = t % 3;
-        const int n = node0 + li;
-        if (n < a.nnodes) {
-            const int64_t o = 3 * (int64_t)n + d;
-            const double body = s_f[li][d];
-            a.body_force[o] = body;
-            const double frc = force_with_bc(body, a.fc_types[o], a.fc_values[o], m.force);
-            a.force[o] = frc;
-            const int bct = a.bc_types[o];
-            const double bcv = a.bc_values[o];
-            double unew;
-            if (a.integrator == PP_EULER) {
-                unew = euler_u(u[o], frc, bct, bcv, m.disp, a.dt);
-            } else {
-                double v = a.ud[o];
-                double acc = a.udd[o];
-                if (a.integrator == PP_EULER_CROMER)
-                    unew = euler_cromer_u(u[o], v, acc, frc, bct, bcv, a.densities[o], m.disp,
-                                          a.damping, a.dt);
-                else
-                    unew = velocity_verlet_u(u[o], v, acc, frc, bct, bcv, a.densities[o],
-                                             m.disp, a.damping, a.dt);
-                a.ud[o] = v;
-                a.udd[o] = acc;
-            }
-            a.u[parity ^ 1][o] = unew;
-        }
-    } else if (t < 4 * wpb) {
-        const int n = node0 + (t - 3 * wpb);
-        if (n < a.nnodes) {
-            const int count = s_cnt[t - 3 * wpb];
-            a.n_neigh[n] = count;
-            a.damage[n] = damage_of(count, a.family[n]);
-        }
-    }
+    f64_node_phase(a, parity, m, node0, wpb, s_f, s_cnt);
 }
 
 // One thread per slot: |r0[j] - r0[i]| as the bond body computes it.
@@ -127,7 +91,7 @@ __global__ void k_bond_lengths(const double* __restrict__ r0, const int32_t* __r
         const double x = dsub(r0[3 * (int64_t)j], r0[3 * i]);
         const double y = dsub(r0[3 * (int64_t)j + 1], r0[3 * i + 1]);
         const double z = dsub(r0[3 * (int64_t)j + 2], r0[3 * i + 2]);
-        len = dsqrt(dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z)));
+        len = f64_length(dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z)));
     }
     length[g] = len;
 }
