@@ -800,9 +800,11 @@ def cpu_block(nx, ny=NY):
         function)
     """
     from probabilistic_peridynamics_gb300 import lattice
+    mod = reference_step_fn()
     coords = lattice.lattice_coords(nx, ny, NZ, DX)
+    # the C restatement takes rows of a power-of-two width
     family, nlist, _ = lattice.lattice_family(nx, ny, NZ, HORIZON_CELLS,
-                                              pow2=False)
+                                              pow2=mod is None)
     n = coords.shape[0]
     bonds = int(family.sum())
     k = lattice.bond_stiffness_pmb(BULK_MODULUS, HORIZON_CELLS * DX)
@@ -815,7 +817,6 @@ def cpu_block(nx, ny=NY):
     # the same strain rate as the full plate: a block nx cells wide is
     # pulled (nx - 1)/(NX - 1) as fast
     rate = PULL_RATE * (nx - 1) / (NX - 1)
-    mod = reference_step_fn()
     if mod is not None:
         nl = compact(nlist, family)
 
