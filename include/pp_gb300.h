@@ -348,6 +348,49 @@ int pp_fused_run(const pp_fused_args* args, int32_t parity, int64_t nsteps,
                  int64_t first, int32_t use_graph, int32_t chunk,
                  int64_t* step_base, void* stream);
 
+/* ------------------------------------------------------------------------ */
+/* PP_FLOAT64 step with each bond computed once: both directions of a bond  */
+/* share its length, stretch and (up to the sign) direction cosines bit for */
+/* bit.  The pair list is built from the neighbour list of the start        */
+/* (pp_pair_count, then pp_pair_fill) and stays valid while bonds only      */
+/* break; the results are those of pp_fused_step.  nnodes * max_neigh must  */
+/* be below 2^31 and npairs below 2^30.                                     */
+/* ------------------------------------------------------------------------ */
+
+typedef struct pp_pairs {
+    int64_t npairs;
+    int32_t symmetric;     /* 1: the two directions' forces are exact
+                              negatives (no bond types, and *differ of
+                              pp_pair_fill is 0)                           */
+    int32_t reserved;      /* must be 0                                    */
+    int32_t* slots;        /* (npairs, 2) the pair's slots; the second is -1
+                              for a pair of one side                       */
+    int32_t* slot_pair;    /* (nnodes, max_neigh) pair of every slot, bit 31
+                              set for its second slot; -1: no bond         */
+    double* length;        /* (npairs) |r0[j] - r0[i]|                     */
+    double* force;         /* (npairs * (symmetric ? 1 : 2), 4) scratch,
+                              32-byte aligned                              */
+} pp_pairs;
+
+/* Counterparts of every slot into slot_pair (nnodes, max_neigh) and the
+ * start of each row's pairs into row_start (nnodes + 1 ints;
+ * row_start[nnodes] = npairs after the stream).  scratch: nnodes ints. */
+int pp_pair_count(const pp_fused_args* args, int32_t* slot_pair, int32_t* row_start,
+                  int32_t* scratch, void* stream);
+
+/* Fills pairs->slots, slot_pair (as pp_pair_count left it) and length.
+ * *differ (a device word) becomes 1 when the two directions of some bond
+ * have other volumes or stiffness corrections. */
+int pp_pair_fill(const pp_fused_args* args, const pp_pairs* pairs, const int32_t* row_start,
+                 int32_t* differ, void* stream);
+
+/* pp_fused_step and pp_fused_run on the pair list. */
+int pp_pair_step(const pp_fused_args* args, const pp_pairs* pairs, int32_t parity,
+                 double displacement_bc_magnitude, double force_bc_magnitude, void* stream);
+int pp_pair_run(const pp_fused_args* args, const pp_pairs* pairs, int32_t parity, int64_t nsteps,
+                const double* disp_mags, const double* force_mags, int64_t first,
+                int32_t use_graph, int32_t chunk, int64_t* step_base, void* stream);
+
 /* Over the bonds (i, j) of nlist (entries != -1): extent[0] = the largest
  * |r0[j][d] - r0[i][d]| over the three components d, extent[1] = the
  * smallest |r0[j] - r0[i]|; extent is two caller-allocated device doubles.

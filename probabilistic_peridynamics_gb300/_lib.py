@@ -102,6 +102,15 @@ class Tiling(ctypes.Structure):
     ]
 
 
+class Pairs(ctypes.Structure):
+    """Mirror of ``pp_pairs``."""
+
+    _fields_ = [
+        ("npairs", _i64), ("symmetric", _i32), ("reserved", _i32),
+        ("slots", _vp), ("slot_pair", _vp), ("length", _vp), ("force", _vp),
+    ]
+
+
 class CorrectionsArgs(ctypes.Structure):
     """Mirror of ``pp_corrections_args``."""
     _fields_ = [
@@ -158,6 +167,17 @@ SIGNATURES = {
         ctypes.c_int,
         [ctypes.POINTER(FusedArgs), _i32, _i64, _vp, _vp, _i64, _i32, _i32,
          _vp, _vp]),
+    "pp_pair_count": (ctypes.c_int, [ctypes.POINTER(FusedArgs), _vp, _vp, _vp,
+                                     _vp]),
+    "pp_pair_fill": (ctypes.c_int, [ctypes.POINTER(FusedArgs),
+                                    ctypes.POINTER(Pairs), _vp, _vp, _vp]),
+    "pp_pair_step": (
+        ctypes.c_int, [ctypes.POINTER(FusedArgs), ctypes.POINTER(Pairs), _i32,
+                       _f64, _f64, _vp]),
+    "pp_pair_run": (
+        ctypes.c_int,
+        [ctypes.POINTER(FusedArgs), ctypes.POINTER(Pairs), _i32, _i64, _vp,
+         _vp, _i64, _i32, _i32, _vp, _vp]),
     "pp_bond_extent": (ctypes.c_int, [_vp, _vp, _i32, _i32, _vp, _vp]),
     "pp_stiffness_corrections": (ctypes.c_int,
                                  [ctypes.POINTER(CorrectionsArgs), _vp]),

@@ -181,16 +181,22 @@ extern "C" int pp_fused_step(const pp_fused_args* args, int32_t parity,
     return launch_fused_step(*args, parity, l, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int pp_fused_run(const pp_fused_args* args, int32_t parity, int64_t nsteps,
-                            const double* disp_mags, const double* force_mags, int64_t first,
-                            int32_t use_graph, int32_t chunk, int64_t* step_base,
+extern "C" int pp_pair_step(const pp_fused_args* args, const pp_pairs* pairs, int32_t parity,
+                            double displacement_bc_magnitude, double force_bc_magnitude,
                             void* stream) {
-    if (!args || (parity != 0 && parity != 1) || nsteps < 0 || first < 0)
-        return PP_ERROR_INVALID_VALUE;
-    if (!disp_mags || !force_mags) return PP_ERROR_INVALID_VALUE;
-    const int v = validate_fused(*args);
-    if (v != PP_SUCCESS || args->nnodes == 0 || nsteps == 0) return v;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!args || !pairs || (parity != 0 && parity != 1)) return PP_ERROR_INVALID_VALUE;
+    const int v = validate_pairs(*args, *pairs);
+    if (v != PP_SUCCESS || args->nnodes == 0) return v;
+    const Launch l{displacement_bc_magnitude, force_bc_magnitude, nullptr, nullptr, nullptr, 0};
+    return launch_pair_step(*args, *pairs, parity, l, static_cast<cudaStream_t>(stream));
+}
+
+// `nsteps` steps, each queued by step(parity, Launch) (a PP_* status), as
+// replays of one graph of `chunk` steps and the rest one by one.
+template <class Step>
+static int run_steps(Step&& step, int32_t parity, int64_t nsteps, const double* disp_mags,
+                     const double* force_mags, int64_t first, int32_t use_graph, int32_t chunk,
+                     int64_t* step_base, cudaStream_t st) {
     int64_t done = 0;
     int p = parity;
     // Graph replay needs a capturable (non-legacy) stream, an even chunk
@@ -206,7 +212,7 @@ extern "C" int pp_fused_run(const pp_fused_args* args, int32_t parity, int64_t n
         int rc = PP_SUCCESS;
         for (int k = 0; k < chunk && rc == PP_SUCCESS; ++k) {
             const Launch l{0.0, 0.0, disp_mags, force_mags, step_base, k};
-            rc = launch_fused_step(*args, p ^ (k & 1), l, st);
+            rc = step(p ^ (k & 1), l);
         }
         if (rc == PP_SUCCESS) {
             k_advance_base<<<1, 1, 0, st>>>(step_base, chunk);
@@ -231,11 +237,40 @@ extern "C" int pp_fused_run(const pp_fused_args* args, int32_t parity, int64_t n
     }
     for (int64_t k = done; k < nsteps; ++k) {
         const Launch l{0.0, 0.0, disp_mags, force_mags, nullptr, first + k};
-        const int rc = launch_fused_step(*args, p, l, st);
+        const int rc = step(p, l);
         if (rc != PP_SUCCESS) return rc;
         p ^= 1;
     }
     return PP_SUCCESS;
+}
+
+extern "C" int pp_fused_run(const pp_fused_args* args, int32_t parity, int64_t nsteps,
+                            const double* disp_mags, const double* force_mags, int64_t first,
+                            int32_t use_graph, int32_t chunk, int64_t* step_base,
+                            void* stream) {
+    if (!args || (parity != 0 && parity != 1) || nsteps < 0 || first < 0)
+        return PP_ERROR_INVALID_VALUE;
+    if (!disp_mags || !force_mags) return PP_ERROR_INVALID_VALUE;
+    const int v = validate_fused(*args);
+    if (v != PP_SUCCESS || args->nnodes == 0 || nsteps == 0) return v;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return run_steps([&](int p, const Launch& l) { return launch_fused_step(*args, p, l, st); },
+                     parity, nsteps, disp_mags, force_mags, first, use_graph, chunk, step_base, st);
+}
+
+extern "C" int pp_pair_run(const pp_fused_args* args, const pp_pairs* pairs, int32_t parity,
+                           int64_t nsteps, const double* disp_mags, const double* force_mags,
+                           int64_t first, int32_t use_graph, int32_t chunk, int64_t* step_base,
+                           void* stream) {
+    if (!args || !pairs || (parity != 0 && parity != 1) || nsteps < 0 || first < 0)
+        return PP_ERROR_INVALID_VALUE;
+    if (!disp_mags || !force_mags) return PP_ERROR_INVALID_VALUE;
+    const int v = validate_pairs(*args, *pairs);
+    if (v != PP_SUCCESS || args->nnodes == 0 || nsteps == 0) return v;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return run_steps(
+        [&](int p, const Launch& l) { return launch_pair_step(*args, *pairs, p, l, st); }, parity,
+        nsteps, disp_mags, force_mags, first, use_graph, chunk, step_base, st);
 }
 
 extern "C" int pp_bond_lengths(const double* r0, const int32_t* nlist, int32_t nnodes,

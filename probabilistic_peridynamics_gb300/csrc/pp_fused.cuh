@@ -38,4 +38,9 @@ int validate_fused(const pp_fused_args& a);
 // Launches one fused step of either precision (pp_fused.cu).
 int launch_fused_step(const pp_fused_args& a, int parity, const Launch& l, cudaStream_t st);
 
+// Argument checks and one step of the pair form (pp_pairs.cu).
+int validate_pairs(const pp_fused_args& a, const pp_pairs& pr);
+int launch_pair_step(const pp_fused_args& a, const pp_pairs& pr, int parity, const Launch& l,
+                     cudaStream_t st);
+
 }  // namespace pp

@@ -34,6 +34,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import check, lib
+from .pairs import DevicePairs, worthwhile
 
 
 class ContextError(Exception):
@@ -406,7 +407,10 @@ class _CUDAIntegrator(Integrator):
         if self.precision == "mixed":
             self._create_mixed_buffers()
         self.bond_length_d = None
-        if self.fused and self.precision == "float64":
+        self._pairs = None
+        pairs = self.fused and self.precision == "float64" and worthwhile(
+            n, mn, int(np.sum(n_neigh)), self.context.device)
+        if self.fused and self.precision == "float64" and not pairs:
             # |xi| per slot, read by the fused binary64 step instead of a
             # square root per bond and step (the same binary64 value)
             self.bond_length_d = torch.empty(
@@ -416,6 +420,9 @@ class _CUDAIntegrator(Integrator):
                 _ptr(self.r0_d), _ptr(self.nlist_d), n, self.max_neighbours,
                 _ptr(self.bond_length_d), self._stream), "pp_bond_lengths")
         self._fargs = self._make_fused_args() if self.fused else None
+        if pairs:
+            self._pairs = DevicePairs(self._fargs, self.context.device,
+                                      self._stream)
         if self.precision == "mixed":
             if self.tiled:
                 from .tiling import DeviceTiling
@@ -550,10 +557,17 @@ class _CUDAIntegrator(Integrator):
             boundary conditions for the current time-step.
         """
         if self.fused:
-            check(lib().pp_fused_step(
-                ctypes.byref(self._fargs), self._parity,
-                float(displacement_bc_magnitude), float(force_bc_magnitude),
-                self._stream), "pp_fused_step")
+            mags = (float(displacement_bc_magnitude),
+                    float(force_bc_magnitude))
+            if self._pairs is not None:
+                check(lib().pp_pair_step(
+                    ctypes.byref(self._fargs),
+                    ctypes.byref(self._pairs.struct), self._parity, *mags,
+                    self._stream), "pp_pair_step")
+            else:
+                check(lib().pp_fused_step(
+                    ctypes.byref(self._fargs), self._parity, *mags,
+                    self._stream), "pp_fused_step")
             self._parity ^= 1
         else:
             self._bond_force(force_bc_magnitude)
@@ -593,10 +607,15 @@ class _CUDAIntegrator(Integrator):
         if not hasattr(self, "_step_base_d"):
             with self.context.on_stream():
                 self._step_base_d = self._zeros((1,), self._torch.int64)
-        check(lib().pp_fused_run(
-            ctypes.byref(self._fargs), self._parity, steps, _ptr(dm),
-            _ptr(fm), first, int(self.use_graph), 16,
-            _ptr(self._step_base_d), self._stream), "pp_fused_run")
+        run = (self._parity, steps, _ptr(dm), _ptr(fm), first,
+               int(self.use_graph), 16, _ptr(self._step_base_d), self._stream)
+        if self._pairs is not None:
+            check(lib().pp_pair_run(
+                ctypes.byref(self._fargs), ctypes.byref(self._pairs.struct),
+                *run), "pp_pair_run")
+        else:
+            check(lib().pp_fused_run(ctypes.byref(self._fargs), *run),
+                  "pp_fused_run")
         self._parity ^= steps & 1
 
     def _bond_force(self, force_bc_magnitude):

@@ -1,0 +1,71 @@
+"""Pair list of the binary64 step (``pp_pairs`` in the C ABI).
+
+Both directions of a bond have the same length, stretch and, up to the sign,
+direction cosines, bit for bit.  With a pair list the step computes each bond
+once (``pp_pair_step``): one kernel over the pairs, one that sums every
+node's slots in the reference's order.  The results are those of
+``pp_fused_step``.
+"""
+import ctypes
+
+from . import _lib
+from ._lib import check, lib
+
+#: Fewest directed bonds for which the pair form is used: below, the second
+#: kernel of a step costs more than the halved bond work saves (one step, one
+#: kernel against pairs: 56,000 bonds 10.0 against 12.3 us, 167,000 bonds 16.4
+#: either way, 273,000 bonds 22.5 against 21.2, 358,000 bonds 26.6 against
+#: 21.5, 1.8M bonds 90 against 62, 42.7M bonds 2,000 against 1,266).
+MIN_BONDS = 250_000
+
+_MAX_SLOTS = 2 ** 31 - 1
+_MAX_PAIRS = 2 ** 30 - 1
+
+
+def worthwhile(nnodes, max_neigh, bonds, device):
+    """Is the pair form used for a model of this size?  ``bonds`` counts the
+    directed bonds.  Its arrays (about 44 bytes a bond) may take half of the
+    device memory that is free, and no more."""
+    import torch
+    slots = nnodes * max_neigh
+    if slots > _MAX_SLOTS or not MIN_BONDS <= bonds <= _MAX_PAIRS:
+        return False
+    free = (torch.cuda.mem_get_info(device)[0]
+            + torch.cuda.memory_reserved(device)
+            - torch.cuda.memory_allocated(device))
+    return 4 * slots + 40 * bonds <= free // 2
+
+
+class DevicePairs:
+    """Device arrays of one pair list, built from the neighbour list (and
+    volumes and corrections) of ``fargs``; queued on ``stream`` (a handle,
+    torch's current stream), which the call waits for."""
+
+    def __init__(self, fargs, device, stream):
+        import torch
+        n, width = int(fargs.nnodes), int(fargs.max_neigh)
+
+        def empty(shape, dtype):
+            return torch.empty(shape, dtype=dtype, device=device)
+
+        args = ctypes.byref(fargs)
+        self.slot_pair = empty((n, width), torch.int32)
+        start = empty((n + 1,), torch.int32)
+        scratch = empty((max(n, 1),), torch.int32)
+        check(lib().pp_pair_count(args, self.slot_pair.data_ptr(),
+                                  start.data_ptr(), scratch.data_ptr(),
+                                  stream), "pp_pair_count")
+        npairs = int(start[n].item())
+        self.slots = empty((max(npairs, 1), 2), torch.int32)
+        self.length = empty((max(npairs, 1),), torch.float64)
+        s = self.struct = _lib.Pairs()
+        s.npairs = npairs
+        s.slots = self.slots.data_ptr()
+        s.slot_pair = self.slot_pair.data_ptr()
+        s.length = self.length.data_ptr()
+        check(lib().pp_pair_fill(args, ctypes.byref(s), start.data_ptr(),
+                                 scratch.data_ptr(), stream), "pp_pair_fill")
+        s.symmetric = int(not fargs.bond_types and scratch[0].item() == 0)
+        self.force = empty((max(npairs, 1) * (1 if s.symmetric else 2), 4),
+                           torch.float64)
+        s.force = self.force.data_ptr()
