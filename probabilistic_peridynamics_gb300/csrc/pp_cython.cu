@@ -106,17 +106,15 @@ __global__ void __launch_bounds__(kWarps * 32)
     if (!__any_sync(kFull, any)) return;  // nothing breaks: the row is unchanged
     __syncwarp();
     int cnt = cnt0;
-    // (1) removals by the lower neighbours, in ascending neighbour index
-    int last = -1;
+    // (1) removals by the lower neighbours, in ascending neighbour index (one
+    // listed twice is removed twice)
     while (true) {
         int best = INT32_MAX;
         for (int p = lane; p < cnt; p += 32)
-            if ((flag[p] & (kLower | kBroken)) == (kLower | kBroken) && row[p] > last &&
-                row[p] < best)
+            if ((flag[p] & (kLower | kBroken)) == (kLower | kBroken) && row[p] < best)
                 best = row[p];
         for (int off = 16; off > 0; off >>= 1) best = min(best, __shfl_xor_sync(kFull, best, off));
         if (best == INT32_MAX) break;
-        last = best;
         int hit = -1;
         for (int p0 = 0; p0 < cnt && hit < 0; p0 += 32) {
             const int p = p0 + lane;
@@ -210,15 +208,17 @@ __global__ void __launch_bounds__(kWarps * 32)
         key[p] = kk;
     }
     __syncwarp();
-    // summation order: rank of each key among the row's keys (keys are
-    // distinct; entries without a bond are left out)
+    // summation order: rank of each key among the row's keys (entries
+    // without a bond are left out)
     int used = 0;
     for (int p = 0; p < cnt; ++p) used += key[p] >= 0;
     for (int p = lane; p < cnt; p += 32) {
         const int kp = key[p];
         if (kp < 0) continue;
         int rank = 0;
-        for (int q = 0; q < cnt; ++q) rank += key[q] >= 0 && key[q] < kp;
+        // (copies of a neighbour listed twice rank in row order)
+        for (int q = 0; q < cnt; ++q)
+            rank += key[q] >= 0 && (key[q] < kp || (key[q] == kp && q < p));
         order[rank] = p;
     }
     __syncwarp();
@@ -312,17 +312,14 @@ __global__ void __launch_bounds__(kWarps * 32)
             str[to] = str[from];
             ref[to] = ref[from];
         };
-        int last = -1;
         while (true) {
             int best = INT32_MAX;
             for (int p = lane; p < cnt; p += 32)
-                if ((flag[p] & (kLower | kBroken)) == (kLower | kBroken) && row[p] > last &&
-                    row[p] < best)
+                if ((flag[p] & (kLower | kBroken)) == (kLower | kBroken) && row[p] < best)
                     best = row[p];
             for (int off = 16; off > 0; off >>= 1)
                 best = min(best, __shfl_xor_sync(kFull, best, off));
             if (best == INT32_MAX) break;
-            last = best;
             int hit = -1;
             for (int p0 = 0; p0 < cnt && hit < 0; p0 += 32) {
                 const int p = p0 + lane;
@@ -390,7 +387,9 @@ __global__ void __launch_bounds__(kWarps * 32)
         const int kp = key[p];
         if (kp < 0) continue;
         int rank = 0;
-        for (int q = 0; q < cnt; ++q) rank += key[q] >= 0 && key[q] < kp;
+        // (copies of a neighbour listed twice rank in row order)
+        for (int q = 0; q < cnt; ++q)
+            rank += key[q] >= 0 && (key[q] < kp || (key[q] == kp && q < p));
         order[rank] = p;
     }
     __syncwarp();
