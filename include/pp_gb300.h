@@ -524,6 +524,52 @@ int pp_cy_break_and_force(const double* coords, const double* u, int32_t* nlist,
 int pp_cy_update_displacement(double* u, const double* bc_values, const int32_t* bc_types,
                               const double* force, double bc_scale, double dt, int32_t nnodes,
                               void* stream);
+/* The whole Euler step with each bond computed once (results of
+ * pp_cy_break_and_force and pp_cy_update_displacement).  The pair list is
+ * built for a symmetric list (pp_cy_check_symmetric): pp_cy_pair_count, then
+ * pp_cy_pair_fill.  nnodes * width below 2^31, npairs below 2^30. */
+typedef struct pp_cy_pairs {
+    int64_t npairs;
+    int32_t symmetric;     /* 1: *differ of pp_cy_pair_fill is 0           */
+    int32_t reserved;      /* must be 0                                    */
+    int32_t* nodes;        /* (npairs, 2) nodes i < j; i < 0 once broken   */
+    int32_t* slot_pair;    /* (nnodes, width) pair of every entry, bit 31
+                              set for a lower neighbour; moves with its
+                              entry; -1: no bond                           */
+    double* length;        /* (npairs) reference lengths                   */
+    double* term;          /* (npairs * (symmetric ? 1 : 2), 4) scratch,
+                              32-byte aligned                              */
+    int32_t* row_state;    /* (nnodes)                                     */
+    double* position;      /* (nnodes, 3) coords + u                       */
+} pp_cy_pairs;
+
+typedef struct pp_cy_step {
+    int32_t nnodes, width;
+    double bond_stiffness, critical_strain, dt;
+    double force_bc_scale, bc_scale;
+    const double* coords;
+    const double* volume;
+    const double* force_bc_values;
+    const int32_t* force_bc_types;
+    const double* bc_values;
+    const int32_t* bc_types;
+    int32_t* nlist;
+    int32_t* n_neigh;
+    double* force;
+    double* u;
+} pp_cy_step;
+
+/* row_state (nnodes) and row_start (nnodes + 1; row_start[nnodes] = npairs
+ * after the stream). */
+int pp_cy_pair_count(const int32_t* nlist, const int32_t* n_neigh, int32_t nnodes, int32_t width,
+                     int32_t* row_state, int32_t* row_start, void* stream);
+/* nodes, slot_pair, length and position; *differ (a device word) becomes 1
+ * when some bond's nodes have other volumes. */
+int pp_cy_pair_fill(const double* coords, const double* u, const double* volume,
+                    const int32_t* nlist, const int32_t* n_neigh, int32_t nnodes, int32_t width,
+                    const int32_t* row_start, const pp_cy_pairs* pairs, int32_t* differ,
+                    void* stream);
+int pp_cy_pair_step(const pp_cy_step* args, const pp_cy_pairs* pairs, void* stream);
 int pp_cy_damage(const int32_t* n_neigh, const int32_t* family, int32_t nnodes, double* damage,
                  void* stream);
 /* The precondition of the calls above, checked on the device before a

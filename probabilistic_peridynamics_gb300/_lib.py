@@ -111,6 +111,29 @@ class Pairs(ctypes.Structure):
     ]
 
 
+class CyPairs(ctypes.Structure):
+    """Mirror of ``pp_cy_pairs``."""
+
+    _fields_ = [
+        ("npairs", _i64), ("symmetric", _i32), ("reserved", _i32),
+        ("nodes", _vp), ("slot_pair", _vp), ("length", _vp), ("term", _vp),
+        ("row_state", _vp), ("position", _vp),
+    ]
+
+
+class CyStep(ctypes.Structure):
+    """Mirror of ``pp_cy_step``."""
+
+    _fields_ = [
+        ("nnodes", _i32), ("width", _i32),
+        ("bond_stiffness", _f64), ("critical_strain", _f64), ("dt", _f64),
+        ("force_bc_scale", _f64), ("bc_scale", _f64),
+        ("coords", _vp), ("volume", _vp), ("force_bc_values", _vp),
+        ("force_bc_types", _vp), ("bc_values", _vp), ("bc_types", _vp),
+        ("nlist", _vp), ("n_neigh", _vp), ("force", _vp), ("u", _vp),
+    ]
+
+
 class CorrectionsArgs(ctypes.Structure):
     """Mirror of ``pp_corrections_args``."""
     _fields_ = [
@@ -198,6 +221,12 @@ SIGNATURES = {
                                              _i32, _vp, _vp, _vp]),
     "pp_cy_update_displacement": (ctypes.c_int, [_vp, _vp, _vp, _vp, _f64,
                                                  _f64, _i32, _vp]),
+    "pp_cy_pair_count": (ctypes.c_int, [_vp, _vp, _i32, _i32, _vp, _vp, _vp]),
+    "pp_cy_pair_fill": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i32,
+                                       _vp, ctypes.POINTER(CyPairs), _vp,
+                                       _vp]),
+    "pp_cy_pair_step": (ctypes.c_int, [ctypes.POINTER(CyStep),
+                                       ctypes.POINTER(CyPairs), _vp]),
     "pp_cy_damage": (ctypes.c_int, [_vp, _vp, _i32, _vp, _vp]),
     "pp_write_sums": (ctypes.c_int, [ctypes.POINTER(WriteSumsArgs), _vp]),
     "pp_mixed_pack": (ctypes.c_int, [ctypes.POINTER(FusedArgs), _i32, _vp]),

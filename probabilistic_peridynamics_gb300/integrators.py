@@ -34,7 +34,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import check, lib
-from .pairs import DevicePairs, worthwhile
+from .pairs import CyPairs, DevicePairs, fits, worthwhile
 
 
 class ContextError(Exception):
@@ -782,10 +782,10 @@ class Euler(Integrator):
 
         :arg float dt: The length of time (in seconds [s]) of one time-step.
         :arg device_context: Optional :class:`CUDAContext` for the kernels.
-        :arg bool fused: True: bond breaking and bond forces in one kernel
-            (``pp_cy_break_and_force``, each bond's strain computed once,
-            reference lengths cached per entry); False: one kernel per
-            Cython function.  Same results.
+        :arg bool fused: True: each bond computed once over a list of pairs
+            (``pp_cy_pair_step``; where that does not fit,
+            ``pp_cy_break_and_force``); False: one kernel per Cython
+            function.  Same results.
         """
         if device_context is not None and not isinstance(device_context,
                                                          CUDAContext):
@@ -894,7 +894,13 @@ class Euler(Integrator):
             self._damage_d = torch.empty(n, dtype=torch.float64,
                                          device=self.device_context.device)
             self._l0_d = None
-            if self.fused and width > 0 and n > 0:
+            self._pairs = None
+            if self.fused and fits(n, width, int(np.sum(n_neigh)),
+                                   self.device_context.device):
+                self._step = self._make_step()
+                self._pairs = CyPairs(self._step, self.device_context.device,
+                                      self.device_context.stream_handle)
+            elif self.fused and width > 0 and n > 0:
                 # reference length of every entry (the same value the step
                 # would compute), kept in entry order by the fused kernel
                 self._l0_d = torch.empty((n, width), dtype=torch.float64,
@@ -903,6 +909,21 @@ class Euler(Integrator):
                     _ptr(self._coords_d), _ptr(self._nlist_d), n, width,
                     _ptr(self._l0_d), self.device_context.stream_handle),
                     "pp_bond_lengths")
+
+    def _make_step(self):
+        a = _lib.CyStep()
+        a.nnodes, a.width = self.nnodes, self._width
+        a.bond_stiffness = float(self.bond_stiffness)
+        a.critical_strain = float(self.critical_stretch)
+        a.dt = float(self.dt)
+        a.coords, a.volume = _ptr(self._coords_d), _ptr(self._volume_d)
+        a.force_bc_values = _ptr(self._fc_values_d)
+        a.force_bc_types = _ptr(self._fc_types_d)
+        a.bc_values = _ptr(self._bc_values_d)
+        a.bc_types = _ptr(self._bc_types_d)
+        a.nlist, a.n_neigh = _ptr(self._nlist_d), _ptr(self._n_neigh_d)
+        a.force, a.u = _ptr(self._force_d), _ptr(self._u_d)
+        return a
 
     def _symmetric(self, nlist_d, n_neigh_d, width):
         """Is j an entry of row i exactly as often as i is one of row j?
@@ -921,6 +942,14 @@ class Euler(Integrator):
         ctx = self.device_context
         st = ctx.stream_handle
         L = lib()
+        if self._pairs is not None:
+            a = self._step
+            a.force_bc_scale = float(force_bc_magnitude)
+            a.bc_scale = float(displacement_bc_magnitude)
+            check(L.pp_cy_pair_step(ctypes.byref(a),
+                                    ctypes.byref(self._pairs.struct), st),
+                  "pp_cy_pair_step")
+            return
         n, w = self.nnodes, self._width
         with ctx.on_stream():
             if self.fused:

@@ -23,12 +23,18 @@ _MAX_PAIRS = 2 ** 30 - 1
 
 
 def worthwhile(nnodes, max_neigh, bonds, device):
-    """Is the pair form used for a model of this size?  ``bonds`` counts the
-    directed bonds.  Its arrays (about 44 bytes a bond) may take half of the
-    device memory that is free, and no more."""
+    """Is the pair form of the fused step used for a model of this size?
+    ``bonds`` counts the directed bonds."""
+    return bonds >= MIN_BONDS and fits(nnodes, max_neigh, bonds, device)
+
+
+def fits(nnodes, max_neigh, bonds, device):
+    """Do the indices and the memory of a pair list fit?  Its arrays (about
+    44 bytes a bond) may take half of the device memory that is free, and no
+    more."""
     import torch
     slots = nnodes * max_neigh
-    if slots > _MAX_SLOTS or not MIN_BONDS <= bonds <= _MAX_PAIRS:
+    if slots > _MAX_SLOTS or bonds > _MAX_PAIRS:
         return False
     free = (torch.cuda.mem_get_info(device)[0]
             + torch.cuda.memory_reserved(device)
@@ -69,3 +75,44 @@ class DevicePairs:
         self.force = empty((max(npairs, 1) * (1 if s.symmetric else 2), 4),
                            torch.float64)
         s.force = self.force.data_ptr()
+
+
+class CyPairs:
+    """Pair list of PeriPy's CPU integrator (``pp_cy_pairs``), built from the
+    compact, symmetric rows of ``step`` (a ``_lib.CyStep``); queued on
+    ``stream``, which the call waits for."""
+
+    def __init__(self, step, device, stream):
+        import torch
+        n, width = int(step.nnodes), int(step.width)
+
+        def empty(shape, dtype):
+            return torch.empty(shape, dtype=dtype, device=device)
+
+        self.row_state = empty((max(n, 1),), torch.int32)
+        start = empty((n + 1,), torch.int32)
+        differ = empty((1,), torch.int32)
+        check(lib().pp_cy_pair_count(step.nlist, step.n_neigh, n, width,
+                                     self.row_state.data_ptr(),
+                                     start.data_ptr(), stream),
+              "pp_cy_pair_count")
+        npairs = int(start[n].item())
+        self.nodes = empty((max(npairs, 1), 2), torch.int32)
+        self.slot_pair = empty((max(n * width, 1),), torch.int32)
+        self.length = empty((max(npairs, 1),), torch.float64)
+        self.position = empty((max(n, 1), 3), torch.float64)
+        s = self.struct = _lib.CyPairs()
+        s.npairs = npairs
+        s.nodes = self.nodes.data_ptr()
+        s.slot_pair = self.slot_pair.data_ptr()
+        s.length = self.length.data_ptr()
+        s.row_state = self.row_state.data_ptr()
+        s.position = self.position.data_ptr()
+        check(lib().pp_cy_pair_fill(
+            step.coords, step.u, step.volume, step.nlist, step.n_neigh, n,
+            width, start.data_ptr(), ctypes.byref(s), differ.data_ptr(),
+            stream), "pp_cy_pair_fill")
+        s.symmetric = int(differ.item() == 0)
+        self.term = empty((max(npairs, 1) * (1 if s.symmetric else 2), 4),
+                          torch.float64)
+        s.term = self.term.data_ptr()
