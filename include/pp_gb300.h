@@ -370,6 +370,10 @@ typedef struct pp_pairs {
     double* length;        /* (npairs) |r0[j] - r0[i]|                     */
     double* force;         /* (npairs * (symmetric ? 1 : 2), 4) scratch,
                               32-byte aligned                              */
+    int32_t* break_step;   /* or NULL: (nnodes, max_neigh), set to `step`
+                              where a bond breaks                          */
+    int32_t step;
+    int32_t reserved2;     /* must be 0                                    */
 } pp_pairs;
 
 /* Counterparts of every slot into slot_pair (nnodes, max_neigh) and the
@@ -712,6 +716,39 @@ int pp_bonds_at_step(const int32_t* nlist0, const int32_t* break_step,
 int pp_adjoint_backward(const pp_adjoint_args* args, const double* u,
                         const double* lam_next, double* lam, double* grad_k,
                         void* stream);
+
+/* A rollout of `steps` Euler steps on a pair list whose pairs all have two
+ * slots (pairs->symmetric 0; args: PP_FLOAT64, PP_EULER, stiffness_corrections
+ * = the per-bond stiffness). */
+typedef struct pp_rollout {
+    int32_t steps;
+    int32_t every;                 /* a checkpoint every so many steps     */
+    const double* mags;            /* HOST: boundary magnitude of each step */
+    double* checkpoints;           /* (ceil(steps / every), nnodes, 3)     */
+    double* states;                /* (every - 1, nnodes, 3) scratch of
+                                      pp_rollout_backward                  */
+    int32_t* break_step;           /* (nnodes, max_neigh): forward: the step
+                                      at which each bond breaks, where one
+                                      does; backward: NULL when none did   */
+} pp_rollout;
+
+/* From args->u[0] to args->u[steps & 1]; args->nlist loses the bonds that
+ * break. */
+int pp_rollout_forward(const pp_fused_args* args, const pp_pairs* pairs, const pp_rollout* r,
+                       void* stream);
+
+/* The reverse of the rollout, its states recomputed segment by segment with
+ * args->critical_stretch (infinite: frozen breaks).  args->nlist (=
+ * adjoint->nlist) holds the bond set of the current step: scratch when
+ * r->break_step is given, else the unbroken list.  lam0 = dL/du_steps; the
+ * result dL/du_0 ends in lam0 or lam1 (steps even or odd).  grad_pair
+ * (npairs, 2), 16-byte aligned, is added to; pp_pair_gradient writes it as
+ * (nnodes, max_neigh). */
+int pp_rollout_backward(const pp_fused_args* args, const pp_pairs* pairs, const pp_rollout* r,
+                        const pp_adjoint_args* adjoint, const int32_t* nlist0, double* lam0,
+                        double* lam1, double* grad_pair, void* stream);
+int pp_pair_gradient(const pp_pairs* pairs, int64_t nslots, const double* grad_pair, double* grad,
+                     void* stream);
 
 /* ------------------------------------------------------------------------ */
 /* Fused steps without any device allocation.                               */

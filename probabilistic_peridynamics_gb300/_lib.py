@@ -108,6 +108,7 @@ class Pairs(ctypes.Structure):
     _fields_ = [
         ("npairs", _i64), ("symmetric", _i32), ("reserved", _i32),
         ("slots", _vp), ("slot_pair", _vp), ("length", _vp), ("force", _vp),
+        ("break_step", _vp), ("step", _i32), ("reserved2", _i32),
     ]
 
 
@@ -157,6 +158,15 @@ class WriteSumsArgs(ctypes.Structure):
         ("body_force", _vp), ("damage", _vp), ("volume", _vp),
         ("plan3", _vp), ("plan1", _vp), ("tip_offsets", _vp),
         ("tip_entries", _vp), ("scratch", _vp), ("sums", _vp),
+    ]
+
+
+class RolloutArgs(ctypes.Structure):
+    """Mirror of ``pp_rollout``."""
+
+    _fields_ = [
+        ("steps", _i32), ("every", _i32), ("mags", _vp),
+        ("checkpoints", _vp), ("states", _vp), ("break_step", _vp),
     ]
 
 
@@ -236,6 +246,15 @@ SIGNATURES = {
     "pp_bonds_at_step": (ctypes.c_int, [_vp, _vp, _i64, _i32, _vp, _vp]),
     "pp_adjoint_backward": (
         ctypes.c_int, [ctypes.POINTER(AdjointArgs), _vp, _vp, _vp, _vp, _vp]),
+    "pp_rollout_forward": (
+        ctypes.c_int, [ctypes.POINTER(FusedArgs), ctypes.POINTER(Pairs),
+                       ctypes.POINTER(RolloutArgs), _vp]),
+    "pp_rollout_backward": (
+        ctypes.c_int, [ctypes.POINTER(FusedArgs), ctypes.POINTER(Pairs),
+                       ctypes.POINTER(RolloutArgs),
+                       ctypes.POINTER(AdjointArgs), _vp, _vp, _vp, _vp, _vp]),
+    "pp_pair_gradient": (ctypes.c_int, [ctypes.POINTER(Pairs), _i64, _vp, _vp,
+                                        _vp]),
     "pp_fused_run_static": (
         ctypes.c_int, [ctypes.POINTER(FusedArgs), _i32, _i64, _vp, _vp, _vp]),
     "pp_static_status": (ctypes.c_int, [_vp, _vp]),

@@ -11,6 +11,11 @@ stiffness corrections with unit bond stiffness, ``peripy/cl/peridynamics.cl
 the first step at which every bond is seen broken is recorded
 (``pp_mark_breaks``), and the state is kept every ``checkpoint_every`` steps.
 
+Where every bond is listed from both ends (as every radius search lists
+them) the steps run on a pair list, queued from C
+(``pp_rollout_forward`` / ``pp_rollout_backward``): the same forward states bit
+for bit, each bond's reverse computed once.
+
 Backward: for each checkpoint segment, last first, the states of the segment
 are recomputed from its checkpoint with the bond set of each step frozen
 (``pp_bonds_at_step``, no new breaks), then ``pp_adjoint_backward`` runs the
@@ -26,6 +31,7 @@ import numpy as np
 from . import _lib
 from ._lib import check, lib
 from .integrators import CUDAContext
+from .pairs import DevicePairs, fits
 
 INT32_MAX = 2 ** 31 - 1
 
@@ -89,19 +95,24 @@ class AdjointProblem:
             check(lib().pp_bond_lengths(_p(self.r0), _p(self.nlist0), n, mn,
                                         _p(self.bond_length), self._stream),
                   "pp_bond_lengths")
+            self.pairs = self._make_pairs()
 
     @property
     def _stream(self):
         return self.context.stream_handle
 
-    def step(self, u, k, t, nlist, critical_stretch):
-        """One binary64 Euler step from ``u``; returns the new state.
+    def _make_pairs(self):
+        """The pair list, or None where some bond is listed from one end
+        only (or the list does not fit)."""
+        bonds = int(self.family.sum().item())
+        if not fits(self.nnodes, self.max_neigh, bonds, self.context.device):
+            return None
+        pairs = DevicePairs(self._fused_args(self.nlist0, None, float("inf")),
+                            self.context.device, self._stream, two_sided=True)
+        return pairs if 2 * pairs.struct.npairs == bonds else None
 
-        ``nlist`` (device, mutated where bonds break) and the per-bond
-        stiffness ``k`` (device float64) define the bonds.
-        """
-        torch = self.torch
-        out = torch.empty_like(u)
+    def _fused_args(self, nlist, k, critical_stretch):
+        """Arguments of a binary64 Euler step (without its states)."""
         a = _lib.FusedArgs()
         a.nnodes, a.max_neigh = self.nnodes, self.max_neigh
         a.integrator, a.precision = _lib.PP_EULER, _lib.PP_FLOAT64
@@ -114,9 +125,92 @@ class AdjointProblem:
         a.stiffness_corrections = _p(k)
         a.bond_length = _p(self.bond_length)
         a.nlist = _p(nlist)
-        a.u[0], a.u[1] = u.data_ptr(), out.data_ptr()
         a.force, a.body_force = _p(self.force), _p(self.body)
         a.n_neigh, a.damage = _p(self.n_neigh), _p(self.damage)
+        return a
+
+    def _adjoint_args(self, nlist, k):
+        a = _lib.AdjointArgs()
+        a.nnodes, a.max_neigh, a.dt = self.nnodes, self.max_neigh, self.dt
+        a.r0, a.vols = _p(self.r0), _p(self.vols)
+        a.nlist, a.partner = _p(nlist), _p(self.partner)
+        a.bc_types, a.stiffness = _p(self.bc_types), _p(k)
+        return a
+
+    def _rollout_args(self, steps, every, checkpoints, break_step,
+                      states=None):
+        r = _lib.RolloutArgs()
+        r.steps, r.every = steps, every
+        self.mags = np.ascontiguousarray(self.mags)
+        r.mags = self.mags.ctypes.data
+        r.checkpoints = _p(checkpoints)
+        r.states = _p(states)
+        r.break_step = _p(break_step)
+        return r
+
+    def run_forward(self, k, steps, every, critical_stretch):
+        """``(u, checkpoints, break_step)`` of a rollout from rest on the
+        pair list: the final state, the state every ``every`` steps and the
+        step at which each slot's bond broke (INT32_MAX: never)."""
+        torch = self.torch
+        if steps:
+            self.mags[steps - 1]  # IndexError where there are too few
+        dev, n = k.device, self.nnodes
+        nl = self.nlist0.clone()
+        breaks = torch.full_like(nl, INT32_MAX)
+        u = [torch.zeros((n, 3), dtype=torch.float64, device=dev),
+             torch.empty((n, 3), dtype=torch.float64, device=dev)]
+        checkpoints = torch.empty((-(-steps // every), n, 3),
+                                  dtype=torch.float64, device=dev)
+        a = self._fused_args(nl, k, critical_stretch)
+        a.u[0], a.u[1] = u[0].data_ptr(), u[1].data_ptr()
+        r = self._rollout_args(steps, every, checkpoints, breaks)
+        check(lib().pp_rollout_forward(
+            ctypes.byref(a), ctypes.byref(self.pairs.struct),
+            ctypes.byref(r), self._stream), "pp_rollout_forward")
+        return u[steps & 1], checkpoints, breaks
+
+    def run_backward(self, grad_u, k, steps, every, checkpoints, breaks):
+        """dL/dk (float64, per slot) from dL/du of the final state."""
+        torch = self.torch
+        broke = bool((breaks != INT32_MAX).any().item())
+        # the bond set of the current step: without breaks, all of them
+        nl = self.nlist0.clone()
+        lam = [grad_u.detach().to(torch.float64).reshape(-1, 3).clone(
+            memory_format=torch.contiguous_format)]
+        lam.append(torch.empty_like(lam[0]))
+        states = torch.empty((max(min(every, steps) - 1, 1), self.nnodes, 3),
+                             dtype=torch.float64, device=k.device)
+        grad_pair = torch.zeros((max(self.pairs.struct.npairs, 1), 2),
+                                dtype=torch.float64, device=k.device)
+        grad_k = torch.empty(self.nlist0.shape, dtype=torch.float64,
+                             device=k.device)
+        a = self._fused_args(nl, k, float("inf"))
+        # (the states of each step are set by the call)
+        a.u[0], a.u[1] = states.data_ptr(), lam[1].data_ptr()
+        r = self._rollout_args(steps, every, checkpoints,
+                               breaks if broke else None, states)
+        pairs = ctypes.byref(self.pairs.struct)
+        check(lib().pp_rollout_backward(
+            ctypes.byref(a), pairs, ctypes.byref(r),
+            ctypes.byref(self._adjoint_args(nl, k)), _p(self.nlist0),
+            _p(lam[0]), _p(lam[1]), _p(grad_pair), self._stream),
+            "pp_rollout_backward")
+        check(lib().pp_pair_gradient(pairs, grad_k.numel(), _p(grad_pair),
+                                     _p(grad_k), self._stream),
+              "pp_pair_gradient")
+        return grad_k
+
+    def step(self, u, k, t, nlist, critical_stretch):
+        """One binary64 Euler step from ``u``; returns the new state.
+
+        ``nlist`` (device, mutated where bonds break) and the per-bond
+        stiffness ``k`` (device float64) define the bonds.
+        """
+        torch = self.torch
+        out = torch.empty_like(u)
+        a = self._fused_args(nlist, k, critical_stretch)
+        a.u[0], a.u[1] = u.data_ptr(), out.data_ptr()
         check(lib().pp_fused_step(ctypes.byref(a), 0, float(self.mags[t]),
                                   0.0, self._stream), "pp_fused_step")
         return out
@@ -130,11 +224,7 @@ class AdjointProblem:
     def backward_step(self, u, lam_next, grad_k, k, nlist):
         torch = self.torch
         lam = torch.empty_like(lam_next)
-        a = _lib.AdjointArgs()
-        a.nnodes, a.max_neigh, a.dt = self.nnodes, self.max_neigh, self.dt
-        a.r0, a.vols = _p(self.r0), _p(self.vols)
-        a.nlist, a.partner = _p(nlist), _p(self.partner)
-        a.bc_types, a.stiffness = _p(self.bc_types), _p(k)
+        a = self._adjoint_args(nlist, k)
         check(lib().pp_adjoint_backward(ctypes.byref(a), _p(u),
                                         _p(lam_next), _p(lam), _p(grad_k),
                                         self._stream), "pp_adjoint_backward")
@@ -155,22 +245,33 @@ def _rollout_function():
             with problem.context.on_stream():
                 k = stiffness.detach().to(torch.float64).contiguous()
                 s0 = float(critical_stretch)
-                nl = problem.nlist0.clone()
-                breaks = torch.full_like(nl, INT32_MAX)
-                u = torch.zeros((problem.nnodes, 3), dtype=torch.float64,
-                                device=k.device)
-                checkpoints = []
-                for t in range(steps):
-                    if t % checkpoint_every == 0:
-                        checkpoints.append(u)
-                    u = problem.step(u, k, t, nl, s0)
-                    check(lib().pp_mark_breaks(_p(nl), _p(breaks), nl.numel(),
-                                               t, problem._stream),
-                          "pp_mark_breaks")
+                # (a pair list takes plain step counts)
+                paired = (problem.pairs is not None
+                          and k.shape == problem.nlist0.shape
+                          and isinstance(steps, int) and steps >= 0
+                          and isinstance(checkpoint_every, int)
+                          and checkpoint_every >= 1)
+                if paired:
+                    u, checkpoints, breaks = problem.run_forward(
+                        k, steps, checkpoint_every, s0)
+                else:
+                    nl = problem.nlist0.clone()
+                    breaks = torch.full_like(nl, INT32_MAX)
+                    u = torch.zeros((problem.nnodes, 3), dtype=torch.float64,
+                                    device=k.device)
+                    checkpoints = []
+                    for t in range(steps):
+                        if t % checkpoint_every == 0:
+                            checkpoints.append(u)
+                        u = problem.step(u, k, t, nl, s0)
+                        check(lib().pp_mark_breaks(
+                            _p(nl), _p(breaks), nl.numel(), t,
+                            problem._stream), "pp_mark_breaks")
             # the caller's stream may use u only after the rollout
             caller.wait_stream(problem.context.stream)
             u.record_stream(caller)
             ctx.problem = problem
+            ctx.paired = paired
             ctx.steps = steps
             ctx.every = checkpoint_every
             ctx.checkpoints = checkpoints
@@ -186,10 +287,17 @@ def _rollout_function():
             caller = torch.cuda.current_stream(problem.context.device)
             problem.context.stream.wait_stream(caller)
             with problem.context.on_stream():
-                lam = grad_u.detach().to(torch.float64).contiguous()
-                grad_k = torch.zeros_like(ctx.k)
-                nl_t = torch.empty_like(problem.nlist0)
-                for seg in reversed(range(len(ctx.checkpoints))):
+                if ctx.paired:
+                    grad_k = problem.run_backward(
+                        grad_u, ctx.k, ctx.steps, ctx.every, ctx.checkpoints,
+                        ctx.breaks)
+                    segments = 0
+                else:
+                    lam = grad_u.detach().to(torch.float64).contiguous()
+                    grad_k = torch.zeros_like(ctx.k)
+                    nl_t = torch.empty_like(problem.nlist0)
+                    segments = len(ctx.checkpoints)
+                for seg in reversed(range(segments)):
                     t0 = seg * ctx.every
                     t1 = min(t0 + ctx.every, ctx.steps)
                     states = [ctx.checkpoints[seg]]

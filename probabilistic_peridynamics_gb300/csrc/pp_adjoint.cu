@@ -16,7 +16,14 @@
 // row m itself: G is the same for both directions of a bond, and the
 // reverse bond's stiffness is found through the partner slot.  One warp per
 // node, no atomics: the gradient is deterministic.
-#include "pp_common.cuh"
+//
+// On a pair list (pp_pairs.cu) whose pairs all have two slots the reverse
+// step computes each bond once: the contribution G v to node m is the negative
+// of the one to node j.  k_adjoint_pairs writes it as a record and adds to
+// both slots' gradients (kept per pair, so that the additions are coalesced;
+// pp_pair_gradient spreads them at the end); k_adjoint_nodes sums the records.
+// A rollout's steps are queued from here (pp_rollout_forward / _backward).
+#include "pp_pairs.cuh"
 
 namespace pp {
 namespace {
@@ -105,6 +112,131 @@ __global__ void __launch_bounds__(kWarps * 32)
     }
 }
 
+constexpr int kPairThreads = 128;
+
+// What a bond's reverse step needs of its geometry: s, 1/|xi|, 1/|p|.
+struct AdjointBond {
+    uint64_t s, inv_xi, inv_y;
+};
+
+static __device__ __noinline__ AdjointBond adjoint_bond_any(double sq, double xi) {
+    using exact64::double_bits;
+    const double y = sqrt(sq);
+    return {double_bits((y - xi) / xi), double_bits(1.0 / xi), double_bits(1.0 / y)};
+}
+
+// On the integer pipe (pp_exact64.cuh) within the limits of f64_stretch.
+__device__ __forceinline__ AdjointBond adjoint_bond(double sq, double xi) {
+    using namespace exact64;
+    const uint64_t sb = double_bits(sq), lb = double_bits(xi);
+    constexpr uint64_t kOne = 0x3FF0000000000000ull;
+    AdjointBond r{0, 0, 0};
+    bool ok = positive_in(sb, 1023 - 400, 1023 + 400) && positive_in(lb, 1023 - 200, 1023 + 200);
+    if (ok) {
+        const Divisor y = sqrt_rn(sb), x = divisor(lb);
+        ok = relative_difference(y, x, r.s);
+        r.inv_y = div_bits(kOne, y);
+        r.inv_xi = div_bits(kOne, x);
+    }
+    if (!ok) r = adjoint_bond_any(sq, xi);
+    return r;
+}
+
+__device__ __forceinline__ d3 free_part(const double* __restrict__ lam,
+                                        const int32_t* __restrict__ bc, int64_t o) {
+    return d3{bc[o] ? 0.0 : lam[o], bc[o + 1] ? 0.0 : lam[o + 1], bc[o + 2] ? 0.0 : lam[o + 2]};
+}
+
+__device__ __forceinline__ double dot(const d3& a, const d3& b) {
+    return __fma_rn(a.x, b.x, __fma_rn(a.y, b.y, a.z * b.z));
+}
+
+// One thread per pair.  Bound by the binary64 pipe: about 45 operations a bond
+// (fused multiply-adds, root and reciprocals on the integer pipe) instead of
+// some 130 from each end, six of them divisions and two square roots.  A pass of the
+// 12,500-node rollout (500 steps forward, recomputed and reversed): 353 ms
+// with k_fused_f64 of the time and k_adjoint_backward, 228 ms after the forward steps'
+// arithmetic moved, 86 ms with both on pairs.
+__global__ void __launch_bounds__(kPairThreads)
+    k_adjoint_pairs(pp_adjoint_args a, pp_pairs pr, int shift, const double* __restrict__ u,
+                    const double* __restrict__ lam_next, double* __restrict__ grad_pair) {
+    __shared__ double s_one;
+    if (threadIdx.x == 0) s_one = 1.0;
+    __syncthreads();
+    const F64Ops op(&s_one);
+    const int64_t q = blockIdx.x * (int64_t)kPairThreads + threadIdx.x;
+    if (q >= pr.npairs) return;
+    const int2 gh = reinterpret_cast<const int2*>(pr.slots)[q];
+    const bool live_g = a.nlist[gh.x] != -1, live_h = a.nlist[gh.y] != -1;
+    if (!live_g && !live_h) return;
+    const int m = gh.x >> shift, j = gh.y >> shift;
+    const int64_t om = 3 * (int64_t)m, oj = 3 * (int64_t)j;
+    F64Bond b{};
+    b.r0 = a.r0;
+    b.u = u;
+    d3 xi;
+    const d3 p = f64_bond_vector(op, b, j, d3{a.r0[om], a.r0[om + 1], a.r0[om + 2]},
+                                 d3{u[om], u[om + 1], u[om + 2]}, xi);
+    const AdjointBond bond = adjoint_bond(dot(p, p), pr.length[q]);
+    const double s = __longlong_as_double(bond.s);
+    const double inv_y = __longlong_as_double(bond.inv_y);
+    const d3 h{p.x * inv_y, p.y * inv_y, p.z * inv_y};
+    const d3 mu_m = free_part(lam_next, a.bc_types, om), mu_j = free_part(lam_next, a.bc_types, oj);
+    const double vol_m = a.vols[m], vol_j = a.vols[j];
+    // v = k_(j,m) vol_m mu_j - k_(m,j) vol_j mu_m over the live directions
+    const double cj = live_h ? a.stiffness[gh.y] * vol_m : 0.0;
+    const double cm = live_g ? a.stiffness[gh.x] * vol_j : 0.0;
+    const d3 v{__fma_rn(cj, mu_j.x, -(cm * mu_m.x)), __fma_rn(cj, mu_j.y, -(cm * mu_m.y)),
+               __fma_rn(cj, mu_j.z, -(cm * mu_m.z))};
+    // G v = (s/|p|) v + (1/|xi| - s/|p|) (h.v) h
+    const double c2 = s * inv_y;
+    const double c1 = (__longlong_as_double(bond.inv_xi) - c2) * dot(h, v);
+    store_record(pr.force + 4 * q, d3{__fma_rn(c2, v.x, c1 * h.x), __fma_rn(c2, v.y, c1 * h.y),
+                                      __fma_rn(c2, v.z, c1 * h.z)});
+    // dL/dk += dt vol s (mu . h), h reversed for the second slot
+    const double t = a.dt * s;
+    double2* g = reinterpret_cast<double2*>(grad_pair) + q;
+    double2 sum = *g;
+    if (live_g) sum.x = __fma_rn(t * vol_j, dot(mu_m, h), sum.x);
+    if (live_h) sum.y = __fma_rn(-(t * vol_m), dot(mu_j, h), sum.y);
+    *g = sum;
+}
+
+// lam = mu + dt (sum of the node's records), one warp per node.
+__global__ void __launch_bounds__(kWarps * 32)
+    k_adjoint_nodes(pp_adjoint_args a, pp_pairs pr, const double* __restrict__ lam_next,
+                    double* __restrict__ lam) {
+    const int lane = threadIdx.x & 31;
+    const int m = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (m >= a.nnodes) return;  // warp-uniform
+    const int64_t row = (int64_t)m * a.max_neigh;
+    d3 v = d3_zero();
+    for (int s = lane; s < a.max_neigh; s += 32) {
+        const int sp = pr.slot_pair[row + s];
+        if (a.nlist[row + s] == -1 || sp == -1) continue;
+        v = d3_add(v, signed_record(pr.force + 4 * (int64_t)(sp & 0x7FFFFFFF), sp));
+    }
+    // packed as in tree_reduce_f64: x on lane 0, z on 8, y on 16
+    const bool up16 = lane & 16, up8 = lane & 8;
+    const double xy = (up16 ? v.y : v.x) + shfl_xor(up16 ? v.x : v.y, 16);
+    const double z = v.z + shfl_xor(v.z, 16);
+    double t = (up8 ? z : xy) + shfl_xor(up8 ? xy : z, 8);
+    for (int off = 4; off >= 1; off >>= 1) t += shfl_xor(t, off);
+    if (lane == 0 || lane == 8 || lane == 16) {
+        const int64_t o = 3 * (int64_t)m + (lane == 0 ? 0 : (lane == 8 ? 2 : 1));
+        lam[o] = __fma_rn(a.dt, t, a.bc_types[o] ? 0.0 : lam_next[o]);
+    }
+}
+
+// The gradient of every slot from those kept per pair (zero elsewhere).
+__global__ void k_pair_gradient(const int32_t* __restrict__ slot_pair, int64_t nslots,
+                                const double* __restrict__ grad_pair, double* __restrict__ grad) {
+    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (g >= nslots) return;
+    const int sp = slot_pair[g];
+    grad[g] = sp == -1 ? 0.0 : grad_pair[2 * (int64_t)(sp & 0x7FFFFFFF) + (sp < 0 ? 1 : 0)];
+}
+
 // First step at which each slot is seen broken.
 __global__ void k_mark_breaks(const int32_t* __restrict__ nlist, int32_t* __restrict__ break_step,
                               int64_t nslots, int32_t t) {
@@ -170,5 +302,114 @@ extern "C" int pp_adjoint_backward(const pp_adjoint_args* args, const double* u,
         return PP_ERROR_INVALID_VALUE;
     k_adjoint_backward<<<(a.nnodes + kWarps - 1) / kWarps, kWarps * 32, 0,
                          static_cast<cudaStream_t>(stream)>>>(a, u, lam_next, lam, grad_k);
+    return launch_status();
+}
+
+namespace pp {
+namespace {
+
+int adjoint_pair_step(const pp_adjoint_args& a, const pp_pairs& pr, const double* u,
+                      const double* lam_next, double* lam, double* grad_pair, cudaStream_t st) {
+    const int shift = 31 - __builtin_clz((unsigned)a.max_neigh);
+    if (pr.npairs > 0)
+        k_adjoint_pairs<<<(unsigned)((pr.npairs + kPairThreads - 1) / kPairThreads), kPairThreads,
+                          0, st>>>(a, pr, shift, u, lam_next, grad_pair);
+    k_adjoint_nodes<<<(a.nnodes + kWarps - 1) / kWarps, kWarps * 32, 0, st>>>(a, pr, lam_next, lam);
+    return launch_status();
+}
+
+int check_rollout(const pp_fused_args* args, const pp_pairs* pairs, const pp_rollout* r) {
+    if (!args || !pairs || !r || r->steps < 0 || r->every < 1) return PP_ERROR_INVALID_VALUE;
+    const int v = validate_pairs(*args, *pairs);
+    if (v != PP_SUCCESS) return v;
+    // each pair's two directions have their own stiffness
+    if (args->integrator != PP_EULER || args->bond_types || pairs->symmetric)
+        return PP_ERROR_INVALID_VALUE;
+    if (r->steps > 0 && (!r->mags || !r->checkpoints)) return PP_ERROR_INVALID_VALUE;
+    return PP_SUCCESS;
+}
+
+Launch at_magnitude(double mag) { return Launch{mag, 0.0, nullptr, nullptr, nullptr, 0}; }
+
+}  // namespace
+}  // namespace pp
+
+extern "C" int pp_rollout_forward(const pp_fused_args* args, const pp_pairs* pairs,
+                                  const pp_rollout* r, void* stream) {
+    const int v = check_rollout(args, pairs, r);
+    if (v != PP_SUCCESS || args->nnodes == 0) return v;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t size = 3 * (size_t)args->nnodes;
+    pp_pairs pr = *pairs;
+    pr.break_step = r->break_step;
+    for (int t = 0; t < r->steps; ++t) {
+        const int p = t & 1;
+        if (t % r->every == 0 &&
+            cudaMemcpyAsync(r->checkpoints + (t / r->every) * size, args->u[p],
+                            size * sizeof(double), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+            return PP_ERROR_CUDA;
+        pr.step = t;
+        const int rc = launch_pair_step(*args, pr, p, at_magnitude(r->mags[t]), st);
+        if (rc != PP_SUCCESS) return rc;
+    }
+    return PP_SUCCESS;
+}
+
+extern "C" int pp_rollout_backward(const pp_fused_args* args, const pp_pairs* pairs,
+                                   const pp_rollout* r, const pp_adjoint_args* adjoint,
+                                   const int32_t* nlist0, double* lam0, double* lam1,
+                                   double* grad_pair, void* stream) {
+    int v = check_rollout(args, pairs, r);
+    if (v != PP_SUCCESS || args->nnodes == 0) return v;
+    if (!adjoint || adjoint->nnodes != args->nnodes || adjoint->max_neigh != args->max_neigh ||
+        adjoint->nlist != args->nlist || !adjoint->r0 || !adjoint->vols || !adjoint->bc_types ||
+        !adjoint->stiffness || !lam0 || !lam1 || lam0 == lam1 || !grad_pair ||
+        (r->every > 1 && !r->states) || (r->break_step && !nlist0) ||
+        (reinterpret_cast<uintptr_t>(grad_pair) & 15u))
+        return PP_ERROR_INVALID_VALUE;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t size = 3 * (size_t)args->nnodes;
+    const int64_t nslots = (int64_t)args->nnodes * args->max_neigh;
+    pp_fused_args a = *args;
+    pp_pairs pr = *pairs;
+    pr.break_step = nullptr;
+    double* lam[2] = {lam0, lam1};
+    int p = 0;
+    // the bond set in force during step t
+    auto bonds = [&](int t) {
+        return r->break_step ? pp_bonds_at_step(nlist0, r->break_step, nslots, t, a.nlist, stream)
+                             : PP_SUCCESS;
+    };
+    for (int t0 = r->steps > 0 ? (r->steps - 1) / r->every * r->every : -1; t0 >= 0;
+         t0 -= r->every) {
+        const int t1 = r->steps - t0 < r->every ? r->steps : t0 + r->every;
+        double* first = r->checkpoints + (t0 / r->every) * size;
+        auto state = [&](int t) { return t == t0 ? first : r->states + (t - t0 - 1) * size; };
+        for (int t = t0; t < t1 - 1; ++t) {
+            if ((v = bonds(t)) != PP_SUCCESS) return v;
+            a.u[0] = state(t);
+            a.u[1] = state(t + 1);
+            if ((v = launch_pair_step(a, pr, 0, at_magnitude(r->mags[t]), st)) != PP_SUCCESS)
+                return v;
+        }
+        for (int t = t1 - 1; t >= t0; --t) {
+            if ((v = bonds(t)) != PP_SUCCESS) return v;
+            if ((v = adjoint_pair_step(*adjoint, pr, state(t), lam[p], lam[p ^ 1], grad_pair,
+                                       st)) != PP_SUCCESS)
+                return v;
+            p ^= 1;
+        }
+    }
+    return PP_SUCCESS;
+}
+
+extern "C" int pp_pair_gradient(const pp_pairs* pairs, int64_t nslots, const double* grad_pair,
+                                double* grad, void* stream) {
+    if (!pairs || nslots < 0) return PP_ERROR_INVALID_VALUE;
+    if (nslots == 0) return PP_SUCCESS;
+    if (!pairs->slot_pair || !grad_pair || !grad) return PP_ERROR_INVALID_VALUE;
+    k_pair_gradient<<<(unsigned)((nslots + 255) / 256), 256, 0,
+                      static_cast<cudaStream_t>(stream)>>>(pairs->slot_pair, nslots, grad_pair,
+                                                           grad);
     return launch_status();
 }

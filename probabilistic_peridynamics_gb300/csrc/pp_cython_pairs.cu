@@ -20,7 +20,7 @@
 //               new position.  A warp's 32 sums advance together, where a
 //               warp per node holds the binary64 pipe for a whole warp per
 //               three sums.
-#include "pp_bond_f64.cuh"
+#include "pp_pairs.cuh"
 
 namespace pp {
 namespace {
@@ -29,7 +29,6 @@ constexpr int kPairThreads = 128;
 constexpr int kBuildWarps = 8;
 constexpr int kRowWarps = 8;  // at most: 48 KB of shared memory a block
 constexpr int kNodeThreads = 192;  // 64 nodes
-constexpr int kReversed = (int)0x80000000u;
 constexpr int kMarked = 1;     // row state: a bond of the row broke this step
 constexpr int kUnordered = 2;  // row state: the entries do not ascend
 
@@ -190,11 +189,6 @@ __global__ void k_cyp_positions(const double* __restrict__ coords, const double*
     if (o < ndof) pos[o] = dadd(coords[o], u[o]);
 }
 
-__device__ __forceinline__ void store_record(double* p, double x, double y, double z, double w) {
-    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w)
-                 : "memory");
-}
-
 // l, strain and fn = strain k / l of a bond of squared length sq.
 struct CyBond {
     uint64_t strain, fn;
@@ -253,10 +247,10 @@ __global__ void __launch_bounds__(kPairThreads, 7)
     const double fn = __longlong_as_double(b.fn);
     const d3 f{op.mul(fn, d.x), op.mul(fn, d.y), op.mul(fn, d.z)};
     const double vj = vol[ij.y];
-    store_record(rec, op.mul(f.x, vj), op.mul(f.y, vj), op.mul(f.z, vj), 0.0);
+    store_record(rec, d3{op.mul(f.x, vj), op.mul(f.y, vj), op.mul(f.z, vj)});
     if constexpr (!SYM) {
         const double vi = vol[ij.x];
-        store_record(rec + 4, op.mul(f.x, vi), op.mul(f.y, vi), op.mul(f.z, vi), 0.0);
+        store_record(rec + 4, d3{op.mul(f.x, vi), op.mul(f.y, vi), op.mul(f.z, vi)});
     }
 }
 

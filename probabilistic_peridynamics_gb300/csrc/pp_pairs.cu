@@ -20,7 +20,7 @@
 // slot that is -1 at a step is dead whoever broke it.  A slot without a
 // counterpart (a one-sided list), the later copies of a neighbour listed
 // twice and a node listed as its own neighbour form pairs of one side.
-#include "pp_bond_f64.cuh"
+#include "pp_pairs.cuh"
 
 namespace pp {
 namespace {
@@ -29,7 +29,6 @@ constexpr int kRowWarps = 8;
 constexpr int kPairThreads = 128;
 constexpr int kSingle = -2;    // build: owner of a pair of one side
 constexpr int kPartner = -3;   // build: the pair's other slot owns it
-constexpr int kReversed = (int)0x80000000u;
 
 // Valid entries of a row that is strictly ascending with its -1 entries at
 // the end; -1 for any other row.  One warp per row.
@@ -182,20 +181,6 @@ __global__ void __launch_bounds__(kRowWarps * 32)
     if (__any_sync(kFull, diff) && lane == 0) atomicOr(differ, 1);
 }
 
-__device__ __forceinline__ void store_record(double* p, const d3& v) {
-    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z),
-                 "d"(0.0)
-                 : "memory");
-}
-
-__device__ __forceinline__ d3 load_record(const double* p) {
-    d3 v;
-    [[maybe_unused]] double w;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(w)
-        : "l"(p));
-    return v;
-}
-
 template <bool CORR, bool TYPES, bool SYM>
 __global__ void __launch_bounds__(kPairThreads, 7)
     k_pair_bonds(pp_fused_args a, pp_pairs pr, int parity, int shift) {
@@ -238,10 +223,12 @@ __global__ void __launch_bounds__(kPairThreads, 7)
         if (live_g && !f64_less(s, a.node_instance ? a.instance_s0[a.node_instance[i]] : b.s0)) {
             live_g = false;
             a.nlist[gh.x] = -1;
+            if (pr.break_step) pr.break_step[gh.x] = pr.step;
         }
         if (live_h && !f64_less(s, a.node_instance ? a.instance_s0[a.node_instance[j]] : b.s0)) {
             live_h = false;
             a.nlist[gh.y] = -1;
+            if (pr.break_step) pr.break_step[gh.y] = pr.step;
         }
         if (!live_g && !live_h) return;
         double f = op.mul(s, b.k);
@@ -253,11 +240,15 @@ __global__ void __launch_bounds__(kPairThreads, 7)
             if (!TYPES && a.node_instance) b.s0 = a.instance_s0[a.node_instance[i]];
             if (f64_bond_law<CORR, TYPES>(op, b, gh.x, s, b.vols[j], f))
                 store_record(pr.force + 8 * p, f64_force(op, f, st));
+            else if (pr.break_step)
+                pr.break_step[gh.x] = pr.step;
         }
         if (live_h) {
             if (!TYPES && a.node_instance) b.s0 = a.instance_s0[a.node_instance[j]];
             if (f64_bond_law<CORR, TYPES>(op, b, gh.y, s, b.vols[i], f))
                 store_record(pr.force + 8 * p + 4, f64_force(op, f, st));
+            else if (pr.break_step)
+                pr.break_step[gh.y] = pr.step;
         }
     }
 }
@@ -285,13 +276,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 5)
                 if (a.nlist[row + k] == -1 || sp == -1) return d3_zero();
                 intact += 1;
                 const int64_t p = sp & 0x7FFFFFFF;
-                const d3 v = load_record(pr.force + (SYM ? 4 * p : 8 * p + (sp < 0 ? 4 : 0)));
-                // by bits: a selected negation is an instruction of the
-                // binary64 pipe
-                const long long flip = sp < 0 ? (long long)0x8000000000000000ull : 0;
-                return d3{__longlong_as_double(__double_as_longlong(v.x) ^ flip),
-                          __longlong_as_double(__double_as_longlong(v.y) ^ flip),
-                          __longlong_as_double(__double_as_longlong(v.z) ^ flip)};
+                return signed_record(pr.force + (SYM ? 4 * p : 8 * p + (sp < 0 ? 4 : 0)), sp);
             });
         const int count = __reduce_add_sync(kFull, intact);
         if (lane == 0) {
@@ -330,7 +315,8 @@ int validate_pairs(const pp_fused_args& a, const pp_pairs& pr) {
     const int v = validate_fused(a);
     if (v != PP_SUCCESS) return v;
     if (a.precision != PP_FLOAT64) return PP_ERROR_UNSUPPORTED;
-    if (pr.npairs < 0 || pr.npairs >= (1ll << 30) || pr.reserved != 0) return PP_ERROR_INVALID_VALUE;
+    if (pr.npairs < 0 || pr.npairs >= (1ll << 30) || pr.reserved != 0 ||
+        pr.reserved2 != 0) return PP_ERROR_INVALID_VALUE;
     if ((int64_t)a.nnodes * a.max_neigh > 0x7FFFFFFFll) return PP_ERROR_UNSUPPORTED;
     if (a.nnodes == 0) return PP_SUCCESS;
     if (!pr.slot_pair || (pr.npairs > 0 && (!pr.slots || !pr.length || !pr.force)))

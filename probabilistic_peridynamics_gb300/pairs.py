@@ -45,9 +45,11 @@ def fits(nnodes, max_neigh, bonds, device):
 class DevicePairs:
     """Device arrays of one pair list, built from the neighbour list (and
     volumes and corrections) of ``fargs``; queued on ``stream`` (a handle,
-    torch's current stream), which the call waits for."""
+    torch's current stream), which the call waits for.  With ``two_sided``
+    each direction of a bond keeps a force of its own, whatever the volumes
+    and corrections."""
 
-    def __init__(self, fargs, device, stream):
+    def __init__(self, fargs, device, stream, two_sided=False):
         import torch
         n, width = int(fargs.nnodes), int(fargs.max_neigh)
 
@@ -71,7 +73,8 @@ class DevicePairs:
         s.length = self.length.data_ptr()
         check(lib().pp_pair_fill(args, ctypes.byref(s), start.data_ptr(),
                                  scratch.data_ptr(), stream), "pp_pair_fill")
-        s.symmetric = int(not fargs.bond_types and scratch[0].item() == 0)
+        s.symmetric = int(not two_sided and not fargs.bond_types
+                          and scratch[0].item() == 0)
         self.force = empty((max(npairs, 1) * (1 if s.symmetric else 2), 4),
                            torch.float64)
         s.force = self.force.data_ptr()
