@@ -806,6 +806,15 @@ int pp_fused_run_static(const pp_fused_args* args, int32_t parity,
 int pp_host_register(void* ptr, size_t bytes);
 int pp_host_unregister(void* ptr);
 
+/* memcpy on several threads (host arrays that do not overlap). */
+int pp_host_copy(void* dst, const void* src, size_t bytes);
+
+/* The first `columns` entries of each of `rows` rows of an int32 neighbour list
+ * of the given width, as int64: entry - offset, and -1 where it is negative
+ * (an instance's rows of a batch in its own numbering). */
+int pp_host_local_rows(const int32_t* src, int64_t rows, int64_t width, int64_t columns,
+                       int64_t offset, int64_t* dst);
+
 /* Copies the status word of the last pp_fused_run_static call on `stream`
  * (PP_STATUS_*) to *status (host memory) and waits for the stream.  No
  * counterpart in the reference. */

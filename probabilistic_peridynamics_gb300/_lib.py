@@ -9,6 +9,8 @@ import ctypes
 import pathlib
 import threading
 
+import numpy as np
+
 _HERE = pathlib.Path(__file__).resolve().parent
 LIB_PATH = _HERE / "libpp_gb300.so"
 
@@ -266,6 +268,8 @@ SIGNATURES = {
                                     ctypes.POINTER(Tiling), _vp]),
     "pp_host_register": (ctypes.c_int, [_vp, ctypes.c_size_t]),
     "pp_host_unregister": (ctypes.c_int, [_vp]),
+    "pp_host_copy": (ctypes.c_int, [_vp, _vp, ctypes.c_size_t]),
+    "pp_host_local_rows": (ctypes.c_int, [_vp, _i64, _i64, _i64, _i64, _vp]),
 }
 
 _lock = threading.Lock()
@@ -292,6 +296,20 @@ def lib():
                 fn.argtypes = args
             _lib = handle
         return _lib
+
+
+#: Host arrays of at least this size are copied on several threads.
+COPY_BYTES = 8 << 20
+
+
+def host_copy(a):
+    """``a.copy()``, a large C-contiguous array on several threads."""
+    if a.nbytes < COPY_BYTES or not a.flags.c_contiguous:
+        return a.copy()
+    out = np.empty_like(a, subok=False)
+    check(lib().pp_host_copy(out.ctypes.data, a.ctypes.data, a.nbytes),
+          "pp_host_copy")
+    return out
 
 
 def check(status, what):

@@ -16,6 +16,8 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
+from ._lib import check, host_copy, lib
+
 
 @dataclass
 class Instance:
@@ -102,7 +104,15 @@ class Batch:
             part = array[a:b]
             if kind == "nlist":
                 w = self.instances[k].nlist.shape[1]
-                part = np.where(part[:, :w] >= 0, part[:, :w] - a, -1)
+                if (part.dtype == np.int32 and part.ndim == 2
+                        and part.flags.c_contiguous):
+                    local = np.empty((b - a, w), dtype=np.int64)
+                    check(lib().pp_host_local_rows(
+                        part.ctypes.data, b - a, part.shape[1], w, a,
+                        local.ctypes.data), "pp_host_local_rows")
+                    part = local
+                else:
+                    part = np.where(part[:, :w] >= 0, part[:, :w] - a, -1)
             out.append(part)
         return out
 
@@ -209,8 +219,8 @@ class BatchedSimulation:
         z = lambda: np.zeros((b.nnodes, 3))  # noqa: E731
         (u, ud, udd, force, body, damage, nlist,
          n_neigh) = self.integrator.write(
-             z(), z(), z(), z(), z(), np.zeros(b.nnodes), b.nlist.copy(),
-             b.n_neigh.copy())
+             z(), z(), z(), z(), z(), np.zeros(b.nnodes),
+             host_copy(b.nlist), b.n_neigh.copy())
         return list(zip(b.split(u), b.split(ud), b.split(damage),
                         b.split(nlist, "nlist"), b.split(n_neigh)))
 

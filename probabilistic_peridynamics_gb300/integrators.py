@@ -101,22 +101,46 @@ def _ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
-#: Host arrays of at least this size are page-locked while a write fills
-#: them from the device.
+#: Host arrays of at least this size are page-locked while they are copied to
+#: or from the device.
 _REGISTER_BYTES = 4 << 20
 
 
-def _pos_frame(coords, extent):
+def _upload(array, dtype, device):
+    """A device tensor of ``array`` as ``dtype``.  A large array is
+    page-locked for the copy (see ``_CUDAIntegrator._put``): 205 MB take 2 ms
+    instead of 11."""
+    import torch
+    a = np.ascontiguousarray(array, dtype=dtype)
+    src = torch.as_tensor(a)
+    if a.nbytes < _REGISTER_BYTES or src.is_pinned():
+        return src.to(device, non_blocking=False)
+    out = torch.empty(a.shape, dtype=src.dtype, device=device)
+    registered = lib().pp_host_register(a.ctypes.data,
+                                        a.nbytes) == _lib.PP_SUCCESS
+    try:
+        out.copy_(src)
+    finally:
+        if registered:
+            lib().pp_host_unregister(a.ctypes.data)
+    return out
+
+
+def _bounds(coords):
+    return coords.min(axis=0), coords.max(axis=0)
+
+
+def _pos_frame(coords, extent, bounds=None):
     """Origin and power-of-two step of the fixed-point positions.
 
     Positions become int32 ``q = rint((r0 - origin) / step)``.  The step is
     the smallest power of two with ``extent / step <= 2**21``, where
     ``extent`` is the largest bond component length, so every bond's
     ``|q[j] - q[i]| < 2**22`` converts to float exactly; it is coarsened if
-    the domain would not fit ``|q| < 2**30``.
+    the domain would not fit ``|q| < 2**30``.  ``bounds``: the smallest and
+    largest coordinates, where they are known already.
     """
-    lo = coords.min(axis=0)
-    hi = coords.max(axis=0)
+    lo, hi = _bounds(coords) if bounds is None else bounds
     origin = (lo + hi) / 2
     half = float(np.max(hi - lo) / 2)
     ext = float(extent) if extent > 0 else max(half, 1.0)
@@ -225,9 +249,7 @@ class _CUDAIntegrator(Integrator):
 
     # -------------------------------------------------------------- helpers
     def _dev(self, array, dtype):
-        import torch
-        t = torch.as_tensor(np.ascontiguousarray(array, dtype=dtype))
-        return t.to(self.context.device, non_blocking=False)
+        return _upload(array, dtype, self.context.device)
 
     def _empty(self, shape, dtype):
         import torch
@@ -299,6 +321,8 @@ class _CUDAIntegrator(Integrator):
             raise ValueError("bond_types shape must be (nnodes, "
                              "max_neighbours)")
         self._torch = torch
+        if self.precision == "mixed":
+            self._coord_bounds = _bounds(self.coords) if self.nnodes else None
         if self.tiled:
             from .tiling import brick_order
             self._order = brick_order(
@@ -432,6 +456,8 @@ class _CUDAIntegrator(Integrator):
                     corrections=self.stiffness_corrections_d is not None,
                     types=self.bond_types_d is not None,
                     instances=self.node_instance_d is not None)
+                # (tiles split to fit the halo capacity stay split)
+                self._order = (self._order[0], self.tiling.tile_start)
                 self._fargs.tiling = ctypes.addressof(self.tiling.struct)
             check(lib().pp_mixed_pack(ctypes.byref(self._fargs), 0,
                                       self._stream), "pp_mixed_pack")
@@ -481,8 +507,8 @@ class _CUDAIntegrator(Integrator):
         ext = ext.cpu().numpy()
         self.bond_extent = float(ext[0])
         self.min_bond = float(ext[1]) if ext[1] < 1e300 else 0.0
-        self.pos_origin, self.pos_scale = _pos_frame(self.coords,
-                                                     self.bond_extent)
+        self.pos_origin, self.pos_scale = _pos_frame(
+            self.coords, self.bond_extent, self._coord_bounds)
 
     def _make_fused_args(self):
         a = _lib.FusedArgs()
@@ -804,11 +830,10 @@ class Euler(Integrator):
         return self._device
 
     def _dev(self, array, dtype, shape=None):
-        import torch
         a = np.ascontiguousarray(array, dtype=dtype)
         if shape is not None:
             a = a.reshape(shape)
-        return torch.as_tensor(a, device=self.device_context.device).clone()
+        return _upload(a, dtype, self.device_context.device)
 
     def build(self, nnodes, degrees_freedom, max_neighbours, coords, volume,
               family, bc_types, bc_values, force_bc_types, force_bc_values,

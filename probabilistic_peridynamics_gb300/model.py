@@ -28,6 +28,7 @@ import warnings
 
 import numpy as np
 
+from ._lib import host_copy
 from .integrators import Integrator
 from .mesh import read_mesh, write_vtk
 
@@ -816,7 +817,7 @@ class Model(object):
                                         force_bc_magnitudes, first_step,
                                         steps)
         if connectivity is None:
-            nlist, n_neigh = (a.copy() for a in self.initial_connectivity)
+            nlist, n_neigh = (host_copy(a) for a in self.initial_connectivity)
         else:
             nlist, n_neigh = _connectivity_pair(connectivity)
         shape = (self.nnodes, self.max_neighbours)

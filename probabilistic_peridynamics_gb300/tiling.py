@@ -123,10 +123,10 @@ class DeviceTiling:
         self.perm = np.ascontiguousarray(perm, dtype=np.int32)
         self.tile_start = np.ascontiguousarray(tile_start, dtype=np.int32)
         n = self.perm.size
-        inv = np.empty(n, dtype=np.int32)
-        inv[self.perm] = np.arange(n, dtype=np.int32)
         self.perm_d = torch.from_numpy(self.perm).to(device)
-        self.inv_d = torch.from_numpy(inv).to(device)
+        self.inv_d = torch.empty_like(self.perm_d)
+        self.inv_d[self.perm_d.long()] = torch.arange(
+            n, dtype=torch.int32, device=device)
         self.struct = _lib.Tiling()
         self.splits = 0
 
