@@ -370,6 +370,7 @@ typedef struct pp_pairs {
     double* length;        /* (npairs) |r0[j] - r0[i]|                     */
     double* force;         /* (npairs * (symmetric ? 1 : 2), 4) scratch,
                               32-byte aligned                              */
+    double* vector;        /* (3, npairs) r0[j] - r0[i]                    */
     int32_t* break_step;   /* or NULL: (nnodes, max_neigh), set to `step`
                               where a bond breaks                          */
     int32_t step;

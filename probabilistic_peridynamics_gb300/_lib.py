@@ -110,7 +110,7 @@ class Pairs(ctypes.Structure):
     _fields_ = [
         ("npairs", _i64), ("symmetric", _i32), ("reserved", _i32),
         ("slots", _vp), ("slot_pair", _vp), ("length", _vp), ("force", _vp),
-        ("break_step", _vp), ("step", _i32), ("reserved2", _i32),
+        ("vector", _vp), ("break_step", _vp), ("step", _i32), ("reserved2", _i32),
     ]
 
 

@@ -171,12 +171,8 @@ __global__ void __launch_bounds__(kPairThreads)
     if (!live_g && !live_h) return;
     const int m = gh.x >> shift, j = gh.y >> shift;
     const int64_t om = 3 * (int64_t)m, oj = 3 * (int64_t)j;
-    F64Bond b{};
-    b.r0 = a.r0;
-    b.u = u;
-    d3 xi;
-    const d3 p = f64_bond_vector(op, b, j, d3{a.r0[om], a.r0[om + 1], a.r0[om + 2]},
-                                 d3{u[om], u[om + 1], u[om + 2]}, xi);
+    const d3 p = f64_deformed(op, u, j, d3{u[om], u[om + 1], u[om + 2]},
+                              pair_reference(pr, q));
     const AdjointBond bond = adjoint_bond(dot(p, p), pr.length[q]);
     const double s = __longlong_as_double(bond.s);
     const double inv_y = __longlong_as_double(bond.inv_y);

@@ -96,30 +96,56 @@ constexpr size_t tree_stack_bytes(int threads) {
 // The last five steps pack the components: a step's lower half computes one
 // component while the upper half computes another (addition commutes, so the
 // sums are the tree's own): 6 additions a warp instead of 15.
-template <int SL, class SlotFn>
+//
+// B slots of a lane are asked for together: slot(k, v) fills v[b] for slots
+// k[b], b < B (a power of two up to SL).  One at a time keeps the registers of
+// long slot code down; four at once keep four loads in flight.
+template <int SL, int B, class SlotFn>
 __device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, int L, double* stack,
                                                   int stride, SlotFn&& slot) {
-    d3 v;
+    static_assert(SL % B == 0, "whole batches");
+    d3 v = d3_zero();
     if constexpr (SL == 1) {
-        v = (lane < L) ? slot(lane) : d3_zero();
+        if (lane < L) {
+            const int k[1] = {lane};
+            d3 one[1];
+            slot(k, one);
+            v = one[0];
+        }
         if (L < 32) {
             for (int off = L >> 1; off >= 1; off >>= 1) v = d3_add(v, d3_shfl_down(v, off));
             const double y = __shfl_sync(kFull, v.y, 0), z = __shfl_sync(kFull, v.z, 0);
             return lane == 0 ? v.x : (lane == 8 ? z : y);
         }
     } else {
+        auto add = [&](const d3& a, const d3& b) {
+            return d3{op.add(a.x, b.x), op.add(a.y, b.y), op.add(a.z, b.z)};
+        };
 #pragma unroll 1
-        for (int n = 0; n < SL; ++n) {
-            v = slot(lane + 32 * static_cast<int>(__brev(n) >> (32 - TreeLevels<SL>::value)));
+        for (int n = 0; n < SL / B; ++n) {
+            int k[B];
+            d3 w[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                k[b] = lane + 32 * static_cast<int>(__brev(n * B + b) >>
+                                                    (32 - TreeLevels<SL>::value));
+            slot(k, w);
+            // the batch's own levels of the tree
+#pragma unroll
+            for (int s = 1; s < B; s <<= 1) {
+#pragma unroll
+                for (int b = 0; b < B; b += 2 * s) w[b] = add(w[b], w[b + s]);
+            }
+            v = w[0];
             double* p = stack;
             int m = n;
 #pragma unroll 1
             while (m & 1) {
-                v = d3{op.add(p[0], v.x), op.add(p[stride], v.y), op.add(p[2 * stride], v.z)};
+                v = add(d3{p[0], p[stride], p[2 * stride]}, v);
                 p += 3 * stride;
                 m >>= 1;
             }
-            if (n != SL - 1) {
+            if (n != SL / B - 1) {
                 p[0] = v.x;
                 p[stride] = v.y;
                 p[2 * stride] = v.z;

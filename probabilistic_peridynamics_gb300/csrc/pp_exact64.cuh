@@ -219,6 +219,45 @@ PP_HD uint64_t pack(uint64_t m, int32_t e) {
     return m + ((uint64_t)(uint32_t)(e - 1) << 52);
 }
 
+// +0 or -0, from the two words: the compiler turns a test of the whole into
+// a comparison on the binary64 pipe.
+PP_HD bool is_zero(uint64_t bits) {
+    uint32_t hi = (uint32_t)(bits >> 32) << 1, lo = (uint32_t)bits;
+#ifdef __CUDA_ARCH__
+    asm("" : "+r"(hi), "+r"(lo));
+#endif
+    return (hi | lo) == 0;
+}
+
+// Rounds hi 2^64 + lo (a product of two 53-bit significands, the first shifted
+// up by 11: 2^115 .. 2^117) to 53 bits, ties to even; e is the product's
+// exponent when hi >= 2^52.  A significand of 2^53 is left as it is: pack()
+// carries it into the exponent.
+PP_HD Num round_product(uint64_t hi, uint64_t lo, int32_t e) {
+    const bool small = (uint32_t)(hi >> 52) == 0;
+    const uint32_t l1 = (uint32_t)(lo >> 32), l0 = (uint32_t)lo;
+    const uint64_t m = small ? (hi << 1) | (l1 >> 31) : hi;
+    const uint32_t f1 = small ? (l1 << 1) | (l0 >> 31) : l1;
+    const uint32_t f0 = small ? l0 << 1 : l0;
+    const uint32_t f = f1 | (uint32_t)(f0 != 0);
+    const uint32_t odd = (uint32_t)m & 1u;
+    return Num{m + (uint64_t)(f > 0x80000000u - odd), e - (int32_t)small};
+}
+
+PP_HD uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+// a a, correctly rounded.
+PP_HD Num square_rn(const Num& a) {
+    const uint64_t s = a.m << 11;
+    const uint32_t a1 = (uint32_t)(s >> 32), a0 = (uint32_t)s;
+    const uint32_t b1 = (uint32_t)(a.m >> 32), b0 = (uint32_t)a.m;
+    const uint64_t p0 = wide(a0, b0);
+    const uint64_t p1 = wide(a1, b0) + (p0 >> 32);
+    const uint64_t p2 = wide(a0, b1) + (uint32_t)p1;
+    const uint64_t hi = wide(a1, b1) + (p1 >> 32) + (p2 >> 32);
+    return round_product(hi, (p2 << 32) | (uint32_t)p0, 2 * a.e - 1022);
+}
+
 // Significand and biased exponent of (a.m 2^a.e) / d, correctly rounded.
 PP_HD Num div_rn(const Num& a, const Divisor& d) {
     const bool lt = a.m < d.m;
@@ -235,16 +274,6 @@ PP_HD Num div_rn(const Num& a, const Divisor& d) {
     return Num{q, a.e - d.e + 1023 - (int32_t)lt};
 }
 
-// +0 or -0, from the two words: the compiler turns a test of the whole into
-// a comparison on the binary64 pipe.
-PP_HD bool is_zero(uint64_t bits) {
-    uint32_t hi = (uint32_t)(bits >> 32) << 1, lo = (uint32_t)bits;
-#ifdef __CUDA_ARCH__
-    asm("" : "+r"(hi), "+r"(lo));
-#endif
-    return (hi | lo) == 0;
-}
-
 // a / d for a of either sign, zero included.  Neither NaN nor infinite; a
 // nonzero a is normal, and so is the quotient (the caller checks).
 PP_HD uint64_t div_bits(uint64_t a, const Divisor& d) {
@@ -252,6 +281,12 @@ PP_HD uint64_t div_bits(uint64_t a, const Divisor& d) {
     const uint64_t sign = a & 0x8000000000000000ull;
     const uint64_t bits = sign | pack(q.m, q.e);
     return is_zero(a) ? a : bits;
+}
+
+// bits of a a (+0 for a zero).
+PP_HD uint64_t square_bits(uint64_t a) {
+    const Num q = square_rn(unpack(a));
+    return is_zero(a) ? 0 : pack(q.m, q.e);
 }
 
 PP_HD double div_signed(uint64_t a, const Divisor& d) { return bits_double(div_bits(a, d)); }

@@ -29,8 +29,7 @@ constexpr int kDefaultWarps = 4;
 // would otherwise occupy GB300's FP64 pipe for a whole warp per 3 lanes).
 template <int SL, bool CORR, bool TYPES>
 __global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parity, Launch l) {
-    __shared__ double s_f[8][3];
-    __shared__ int s_cnt[8];
+    __shared__ NodeStage stage;
     __shared__ double s_one;
     extern __shared__ double s_stack[];
     if (threadIdx.x == 0) s_one = 1.0;
@@ -41,6 +40,7 @@ __global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parit
     const int warp = threadIdx.x >> 5;
     const int node0 = blockIdx.x * wpb;
     const int i = node0 + warp;
+    f64_stage_nodes(a, parity, node0, wpb, stage);
     const StepMags m = step_mags(l);
     const double* __restrict__ u = a.u[parity];
     if (i < a.nnodes) {  // warp-uniform
@@ -63,20 +63,20 @@ __global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parit
         const d3 ui{u[o3], u[o3 + 1], u[o3 + 2]};
         const int64_t row = (int64_t)i * a.max_neigh;
         int intact = 0;
-        const double f = tree_reduce_f64<SL>(op, lane, a.max_neigh, s_stack + threadIdx.x,
-                                             blockDim.x, [&](int k) {
-            return f64_slot<CORR, TYPES>(op, b, row + k, ri, ui, intact);
-        });
+        const double f = tree_reduce_f64<SL, 1>(
+            op, lane, a.max_neigh, s_stack + threadIdx.x, blockDim.x,
+            [&](const int(&k)[1], d3(&v)[1]) {
+                v[0] = f64_slot<CORR, TYPES>(op, b, row + k[0], ri, ui, intact);
+            });
         const int count = __reduce_add_sync(kFull, intact);
         if (lane == 0) {
-            s_f[warp][0] = f;
-            s_cnt[warp] = count;
+            stage.sum[3 * warp] = f;
+            stage.count[warp] = count;
         }
-        if (lane == 16) s_f[warp][1] = f;
-        if (lane == 8) s_f[warp][2] = f;
+        if (lane == 16) stage.sum[3 * warp + 1] = f;
+        if (lane == 8) stage.sum[3 * warp + 2] = f;
     }
-    __syncthreads();
-    f64_node_phase(a, parity, m, node0, wpb, s_f, s_cnt);
+    f64_node_phase(a, parity, m, node0, wpb, stage);
 }
 
 // One thread per slot: |r0[j] - r0[i]| as the bond body computes it.

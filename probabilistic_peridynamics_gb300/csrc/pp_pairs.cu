@@ -12,9 +12,13 @@
 //  k_pair_nodes  one warp per node: the records of its slots summed in the
 //                work-group tree order (pp_common.cuh), then the node update.
 //
-// The per-bond work is bound by the binary64 and integer pipes, so halving
-// it outweighs writing and gathering the records (32 bytes a pair written,
-// 32 gathered per slot).
+// Both kernels are bound by the binary64 pipe (87 and 89 % busy on the plate of
+// 400,000 nodes in rows of 128 slots: 0.63 + 0.39 ms), so halving the bond
+// work (1.95 ms in one kernel) outweighs writing and gathering the records (32 bytes
+// a pair written, 32 gathered per slot).  What that pipe does not have to do is
+// kept off it: roots and quotients (pp_exact64.cuh), the reference vectors
+// (24 bytes a pair read instead of three subtractions, 0.66 -> 0.63 ms), signs
+// and selects.
 //
 // The pair list depends only on the bonds that exist when it is built; a
 // slot that is -1 at a step is dead whoever broke it.  A slot without a
@@ -170,6 +174,9 @@ __global__ void __launch_bounds__(kRowWarps * 32)
             const double y = dsub(r0[3 * (int64_t)j + 1], r0[o + 1]);
             const double z = dsub(r0[3 * (int64_t)j + 2], r0[o + 2]);
             pr.length[p] = f64_length(dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z)));
+            pr.vector[p] = x;
+            pr.vector[pr.npairs + p] = y;
+            pr.vector[2 * pr.npairs + p] = z;
             if (v >= 0) {
                 pr.slot_pair[v] = p | kReversed;
                 diff |= __double_as_longlong(vols[i]) != __double_as_longlong(vols[j]);
@@ -182,7 +189,7 @@ __global__ void __launch_bounds__(kRowWarps * 32)
 }
 
 template <bool CORR, bool TYPES, bool SYM>
-__global__ void __launch_bounds__(kPairThreads, 7)
+__global__ void __launch_bounds__(kPairThreads, 8)
     k_pair_bonds(pp_fused_args a, pp_pairs pr, int parity, int shift) {
     __shared__ double s_one;
     if (threadIdx.x == 0) s_one = 1.0;
@@ -211,11 +218,9 @@ __global__ void __launch_bounds__(kPairThreads, 7)
               a.critical_stretch,
               a.nregimes};
     const int64_t oi = 3 * (int64_t)i;
-    const d3 ri{b.r0[oi], b.r0[oi + 1], b.r0[oi + 2]};
     const d3 ui{b.u[oi], b.u[oi + 1], b.u[oi + 2]};
-    d3 xi;
-    const d3 xe = f64_bond_vector(op, b, j, ri, ui, xi);
-    const F64Stretch st = f64_stretch(xe.x, xe.y, xe.z, f64_square(op, xe), pr.length[p]);
+    const d3 xe = f64_deformed(op, b.u, j, ui, pair_reference(pr, p));
+    const F64Stretch st = f64_stretch<false>(op, xe, pr.length[p]);
     bool live_g = jg != -1, live_h = jh != -1;
     const double s = __longlong_as_double(st.s);
     if constexpr (SYM) {
@@ -253,11 +258,14 @@ __global__ void __launch_bounds__(kPairThreads, 7)
     }
 }
 
+// Latency-bound until four slots' loads are in flight and the node updates'
+// inputs are staged (0.56 -> 0.43 ms); then 32 registers, so that 64 warps
+// are resident (0.39 ms; rows of 256 slots hold more and do better with 48:
+// 0.354 against 0.369 ms a step at 68,000 nodes).
 template <int SL, bool SYM>
-__global__ void __launch_bounds__(kRowWarps * 32, 5)
+__global__ void __launch_bounds__(kRowWarps * 32, SL <= 4 ? 8 : 6)
     k_pair_nodes(pp_fused_args a, pp_pairs pr, int parity, Launch l) {
-    __shared__ double s_f[kRowWarps][3];
-    __shared__ int s_cnt[kRowWarps];
+    __shared__ NodeStage stage;
     __shared__ double s_one;
     extern __shared__ double s_stack[];
     if (threadIdx.x == 0) s_one = 1.0;
@@ -267,27 +275,38 @@ __global__ void __launch_bounds__(kRowWarps * 32, 5)
     const int warp = threadIdx.x >> 5;
     const int node0 = blockIdx.x * kRowWarps;
     const int i = node0 + warp;
+    f64_stage_nodes(a, parity, node0, kRowWarps, stage);
     if (i < a.nnodes) {  // warp-uniform
         const int64_t row = (int64_t)i * a.max_neigh;
         int intact = 0;
-        const double f = tree_reduce_f64<SL>(
-            op, lane, a.max_neigh, s_stack + threadIdx.x, kRowWarps * 32, [&](int k) {
-                const int sp = pr.slot_pair[row + k];
-                if (a.nlist[row + k] == -1 || sp == -1) return d3_zero();
-                intact += 1;
-                const int64_t p = sp & 0x7FFFFFFF;
-                return signed_record(pr.force + (SYM ? 4 * p : 8 * p + (sp < 0 ? 4 : 0)), sp);
+        constexpr int kBatch = SL < 4 ? SL : 4;
+        const double f = tree_reduce_f64<SL, kBatch>(
+            op, lane, a.max_neigh, s_stack + threadIdx.x, kRowWarps * 32,
+            [&](const int(&k)[kBatch], d3(&v)[kBatch]) {
+                // all indices of a batch, then all its records
+                int sp[kBatch];
+#pragma unroll
+                for (int b = 0; b < kBatch; ++b) {
+                    sp[b] = pr.slot_pair[row + k[b]];
+                    if (a.nlist[row + k[b]] == -1) sp[b] = -1;
+                }
+#pragma unroll
+                for (int b = 0; b < kBatch; ++b) {
+                    intact += sp[b] != -1;
+                    const int64_t p = sp[b] & 0x7FFFFFFF;
+                    v[b] = signed_record(pr.force + (SYM ? 4 * p : 8 * p + (sp[b] < 0 ? 4 : 0)),
+                                         sp[b]);
+                }
             });
         const int count = __reduce_add_sync(kFull, intact);
         if (lane == 0) {
-            s_f[warp][0] = f;
-            s_cnt[warp] = count;
+            stage.sum[3 * warp] = f;
+            stage.count[warp] = count;
         }
-        if (lane == 16) s_f[warp][1] = f;
-        if (lane == 8) s_f[warp][2] = f;
+        if (lane == 16) stage.sum[3 * warp + 1] = f;
+        if (lane == 8) stage.sum[3 * warp + 2] = f;
     }
-    __syncthreads();
-    f64_node_phase(a, parity, step_mags(l), node0, kRowWarps, s_f, s_cnt);
+    f64_node_phase(a, parity, step_mags(l), node0, kRowWarps, stage);
 }
 
 template <bool CORR, bool TYPES, bool SYM>
@@ -319,7 +338,7 @@ int validate_pairs(const pp_fused_args& a, const pp_pairs& pr) {
         pr.reserved2 != 0) return PP_ERROR_INVALID_VALUE;
     if ((int64_t)a.nnodes * a.max_neigh > 0x7FFFFFFFll) return PP_ERROR_UNSUPPORTED;
     if (a.nnodes == 0) return PP_SUCCESS;
-    if (!pr.slot_pair || (pr.npairs > 0 && (!pr.slots || !pr.length || !pr.force)))
+    if (!pr.slot_pair || (pr.npairs > 0 && (!pr.slots || !pr.length || !pr.vector || !pr.force)))
         return PP_ERROR_INVALID_VALUE;
     if (pr.symmetric && a.bond_types) return PP_ERROR_INVALID_VALUE;
     if (!aligned32(pr.force) || (reinterpret_cast<uintptr_t>(pr.slots) & 7u)) return PP_ERROR_MISALIGNED;
@@ -399,7 +418,7 @@ extern "C" int pp_pair_fill(const pp_fused_args* args, const pp_pairs* pairs,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(differ, 0, sizeof(int32_t), st) != cudaSuccess) return PP_ERROR_CUDA;
     if (a.nnodes == 0) return PP_SUCCESS;
-    if (!row_start || !pairs->slot_pair || (pairs->npairs > 0 && (!pairs->slots || !pairs->length)))
+    if (!row_start || !pairs->slot_pair || (pairs->npairs > 0 && (!pairs->slots || !pairs->length || !pairs->vector)))
         return PP_ERROR_INVALID_VALUE;
     k_pair_fill<<<(unsigned)((a.nnodes + kRowWarps - 1) / kRowWarps), kRowWarps * 32, 0, st>>>(
         a.nlist, a.r0, a.vols, a.stiffness_corrections, a.nnodes, a.max_neigh, row_start, *pairs,

@@ -13,19 +13,29 @@ __device__ __forceinline__ void store_record(double* p, const d3& v) {
                  : "memory");
 }
 
-__device__ __forceinline__ d3 load_record(const double* p) {
-    d3 v;
-    [[maybe_unused]] double w;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(w)
-        : "l"(p));
+// Reference vector of pair p, r0[j] - r0[i] as pp_pair_fill kept it.
+__device__ __forceinline__ d3 pair_reference(const pp_pairs& pr, int64_t p) {
+    return d3{pr.vector[p], pr.vector[pr.npairs + p], pr.vector[2 * pr.npairs + p]};
+}
+
+// The record at p where `live`, else +0 (without a branch around the load).
+__device__ __forceinline__ d3 load_record_if(const double* p, bool live) {
+    d3 v{0.0, 0.0, 0.0};
+    [[maybe_unused]] double w = 0.0;
+    asm("{\n\t.reg .pred live;\n\t"
+        "setp.ne.s32 live, %5, 0;\n\t"
+        "@live ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+d"(v.x), "+d"(v.y), "+d"(v.z), "+d"(w)
+        : "l"(p), "r"((int)live));
     return v;
 }
 
-// The record at p as slot `sp` sees it: negated for a pair's second slot.  By
-// bits: a selected negation is an instruction of the binary64 pipe.
+// The record at p as slot `sp` sees it: negated for a pair's second slot, +0
+// for sp = -1.  By bits: a selected negation is an instruction of the
+// binary64 pipe.
 __device__ __forceinline__ d3 signed_record(const double* p, int sp) {
-    const d3 v = load_record(p);
-    const long long flip = sp < 0 ? (long long)0x8000000000000000ull : 0;
+    const d3 v = load_record_if(p, sp != -1);
+    const long long flip = sp < -1 ? (long long)0x8000000000000000ull : 0;
     return d3{__longlong_as_double(__double_as_longlong(v.x) ^ flip),
               __longlong_as_double(__double_as_longlong(v.y) ^ flip),
               __longlong_as_double(__double_as_longlong(v.z) ^ flip)};

@@ -42,9 +42,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     const d3 ui{a.u[3 * (int64_t)i], a.u[3 * (int64_t)i + 1], a.u[3 * (int64_t)i + 2]};
     const int64_t row = (int64_t)i * a.max_neigh;
     int intact = 0;
-    const double f = tree_reduce_f64<SL>(
+    const double f = tree_reduce_f64<SL, 1>(
         op, lane, a.max_neigh, s_stack + threadIdx.x, kWarpsPerBlock * 32,
-        [&](int k) { return f64_slot<CORR, TYPES>(op, b, row + k, ri, ui, intact); });
+        [&](const int(&k)[1], d3(&v)[1]) {
+            v[0] = f64_slot<CORR, TYPES>(op, b, row + k[0], ri, ui, intact);
+        });
     if (lane == 0 || lane == 8 || lane == 16) {  // x, z, y
         const int64_t o = 3 * (int64_t)i + (lane == 0 ? 0 : (lane == 8 ? 2 : 1));
         a.body_force[o] = f;

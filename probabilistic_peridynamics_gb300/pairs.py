@@ -13,9 +13,9 @@ from ._lib import check, lib
 
 #: Fewest directed bonds for which the pair form is used: below, the second
 #: kernel of a step costs more than the halved bond work saves (one step, one
-#: kernel against pairs: 56,000 bonds 10.0 against 12.3 us, 167,000 bonds 16.4
-#: either way, 273,000 bonds 22.5 against 21.2, 358,000 bonds 26.6 against
-#: 21.5, 1.8M bonds 90 against 62, 42.7M bonds 2,000 against 1,266).
+#: kernel against pairs: 56,000 bonds 8.2 against 12.3 us, 167,000 bonds 16.4
+#: against 16.2, 273,000 bonds 22.5 against 21.2, 1.8M bonds 88 against 53,
+#: 42.7M bonds 1,950 against 1,020).
 MIN_BONDS = 250_000
 
 _MAX_SLOTS = 2 ** 31 - 1
@@ -29,9 +29,9 @@ def worthwhile(nnodes, max_neigh, bonds, device):
 
 
 def fits(nnodes, max_neigh, bonds, device):
-    """Do the indices and the memory of a pair list fit?  Its arrays (about
-    44 bytes a bond) may take half of the device memory that is free, and no
-    more."""
+    """Do the indices and the memory of a pair list fit?  Its arrays (four
+    bytes a slot and up to 52 a bond) may take half of the device memory that
+    is free, and no more."""
     import torch
     slots = nnodes * max_neigh
     if slots > _MAX_SLOTS or bonds > _MAX_PAIRS:
@@ -39,7 +39,7 @@ def fits(nnodes, max_neigh, bonds, device):
     free = (torch.cuda.mem_get_info(device)[0]
             + torch.cuda.memory_reserved(device)
             - torch.cuda.memory_allocated(device))
-    return 4 * slots + 40 * bonds <= free // 2
+    return 4 * slots + 52 * bonds <= free // 2
 
 
 class DevicePairs:
@@ -66,11 +66,13 @@ class DevicePairs:
         npairs = int(start[n].item())
         self.slots = empty((max(npairs, 1), 2), torch.int32)
         self.length = empty((max(npairs, 1),), torch.float64)
+        self.vector = empty((3, max(npairs, 1)), torch.float64)
         s = self.struct = _lib.Pairs()
         s.npairs = npairs
         s.slots = self.slots.data_ptr()
         s.slot_pair = self.slot_pair.data_ptr()
         s.length = self.length.data_ptr()
+        s.vector = self.vector.data_ptr()
         check(lib().pp_pair_fill(args, ctypes.byref(s), start.data_ptr(),
                                  scratch.data_ptr(), stream), "pp_pair_fill")
         s.symmetric = int(not two_sided and not fargs.bond_types

@@ -1,4 +1,4 @@
-"""The binary64 roots and quotients of ``csrc/pp_exact64.cuh`` on the CPU.
+"""The binary64 roots, quotients and squares of ``csrc/pp_exact64.cuh`` on the CPU.
 
 The header also compiles for the host; every result must equal NumPy's
 (correctly rounded) ``sqrt`` and division bit for bit, with the FP32 seeds
@@ -21,13 +21,14 @@ SHIM = """
 using namespace pp::exact64;
 extern "C" void run(long n, float shift, const double* a, const double* b,
                     double* root, double* quotient, double* stretch,
-                    int* fits) {
+                    double* square, int* fits) {
     seed_shift() = shift;
     for (long i = 0; i < n; ++i) {
         const Divisor y = sqrt_rn(double_bits(a[i] < 0 ? -a[i] : a[i]));
         root[i] = bits_double(pack(y.m, y.e));
         const Divisor d = divisor(double_bits(b[i]));
         quotient[i] = div_signed(double_bits(a[i]), d);
+        square[i] = bits_double(square_bits(double_bits(b[i])));
         uint64_t s = 0;
         const Divisor p = divisor(double_bits(a[i] < 0 ? -a[i] : a[i]));
         fits[i] = relative_difference(p, d, s);
@@ -65,7 +66,7 @@ def _numbers(rng, n, lo, hi):
 
 def _run(shim, a, b, shift):
     a, b = (np.ascontiguousarray(x, dtype=np.float64) for x in (a, b))
-    out = [np.empty_like(a) for _ in range(3)]
+    out = [np.empty_like(a) for _ in range(4)]
     fits = np.empty(a.size, dtype=np.int32)
     p = [x.ctypes.data_as(ctypes.c_void_p) for x in (a, b, *out, fits)]
     shim.run(ctypes.c_long(a.size), ctypes.c_float(shift), *p)
@@ -92,9 +93,10 @@ def test_bits(shim, shift, case):
     else:
         a = np.zeros(n)
         b[:100] = 1.0
-    root, quotient, stretch, fits = _run(shim, a, b, shift)
+    root, quotient, stretch, square, fits = _run(shim, a, b, shift)
     expect = a / b
     assert np.array_equal(quotient.view(np.uint64), expect.view(np.uint64))
+    assert np.array_equal(square.view(np.uint64), (b * b).view(np.uint64))
     if case == "zero":
         return
     expect = np.sqrt(np.abs(a))

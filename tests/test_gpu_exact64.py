@@ -26,7 +26,8 @@ CASES = {"ordinary": (1.0, 1e-3, 0),
          "stretched": (1.0, 5.0, 0),
          "squeezed": (1.0, -0.45, 0),
          "subnormal": (1.0, 1e-309, 1),
-         "tiny": (1.0, 1e-215, 1)}
+         "small": (1.0, 1e-140, 1),
+         "tiny": (1.0, 1e-155, 1)}
 
 
 @pytest.mark.parametrize("fused", [True, False])
