@@ -11,31 +11,42 @@ import ctypes
 from . import _lib
 from ._lib import check, lib
 
-#: Fewest directed bonds for which the pair form is used: below, the second
-#: kernel of a step costs more than the halved bond work saves (one step, one
-#: kernel against pairs: 56,000 bonds 8.2 against 12.3 us, 167,000 bonds 16.4
-#: against 16.2, 273,000 bonds 22.5 against 21.2, 1.8M bonds 88 against 53,
-#: 42.7M bonds 1,950 against 1,020).
-MIN_BONDS = 250_000
+#: Rows of at most this many slots are one load a lane in the one-kernel step,
+#: which a second kernel beats only from ``MIN_BONDS`` directed bonds (one step,
+#: one kernel against pairs: 23,000 bonds 5.4 against 6.8 us, 56,000 bonds 6.7
+#: against 7.7, 97,000 bonds 8.0 against 8.6, 173,000 bonds 13.4 against 10.8,
+#: 3.5M bonds 268 against 223).  Wider rows are a serial loop over their slots
+#: there, so pairs are faster at every size (rows of 64: 39,000 bonds 7.9
+#: against 6.9 us, 94,000 bonds 10.2 against 8.7; rows of 128: 6,800 bonds 10.1
+#: against 7.4, 167,000 bonds 14.6 against 10.5, 2.9M bonds 139 against 80,
+#: 42.7M bonds 1,950 against 1,010; rows of 256: 121,000 bonds 18.8 against
+#: 10.5, 3.6M bonds 153 against 95).
+NARROW = 32
+MIN_BONDS = 150_000
 
 _MAX_SLOTS = 2 ** 31 - 1
 _MAX_PAIRS = 2 ** 30 - 1
+_SMALL_BYTES = 2 ** 25
 
 
 def worthwhile(nnodes, max_neigh, bonds, device):
     """Is the pair form of the fused step used for a model of this size?
     ``bonds`` counts the directed bonds."""
-    return bonds >= MIN_BONDS and fits(nnodes, max_neigh, bonds, device)
+    return ((max_neigh > NARROW or bonds >= MIN_BONDS)
+            and fits(nnodes, max_neigh, bonds, device))
 
 
 def fits(nnodes, max_neigh, bonds, device):
     """Do the indices and the memory of a pair list fit?  Its arrays (four
     bytes a slot and up to 52 a bond) may take half of the device memory that
-    is free, and no more."""
+    is free, and no more; of a small list that is not asked (it takes longer
+    than building the list)."""
     import torch
     slots = nnodes * max_neigh
     if slots > _MAX_SLOTS or bonds > _MAX_PAIRS:
         return False
+    if 4 * slots + 52 * bonds <= _SMALL_BYTES:
+        return True
     free = (torch.cuda.mem_get_info(device)[0]
             + torch.cuda.memory_reserved(device)
             - torch.cuda.memory_allocated(device))

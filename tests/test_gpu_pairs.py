@@ -66,10 +66,10 @@ def _model(form, kind):
     return s, more
 
 
-def _run(monkeypatch, form, kind, threshold, steps):
+def _run(monkeypatch, form, kind, pairs, steps):
     import probabilistic_peridynamics_gb300 as pp
-    from probabilistic_peridynamics_gb300 import pairs
-    monkeypatch.setattr(pairs, "MIN_BONDS", threshold)
+    from probabilistic_peridynamics_gb300 import integrators
+    monkeypatch.setattr(integrators, "worthwhile", lambda *_: pairs)
     s, more = _model(form, kind)
     cls = {"euler": pp.EulerCUDA, "euler_cromer": pp.EulerCromerCUDA,
            "velocity_verlet": pp.VelocityVerletCUDA}[kind]
@@ -79,14 +79,14 @@ def _run(monkeypatch, form, kind, threshold, steps):
         integ.set_instances(half, np.array([s["s0"], 0.6 * s["s0"]]))
     out = run_integrator(integ, s, steps, 3e-3 * np.arange(1, steps + 1),
                          force_mags=np.zeros(steps), use_run=True, **more)
-    assert (integ._pairs is not None) == (threshold == 0)
+    assert (integ._pairs is not None) == pairs
     return out, s
 
 
 @pytest.mark.parametrize("form", FORMS)
 def test_same_bits(monkeypatch, form):
-    one, s = _run(monkeypatch, form, "velocity_verlet", 2 ** 40, 50)
-    two, _ = _run(monkeypatch, form, "velocity_verlet", 0, 50)
+    one, s = _run(monkeypatch, form, "velocity_verlet", False, 50)
+    two, _ = _run(monkeypatch, form, "velocity_verlet", True, 50)
     for a, b in zip(one, two):
         assert np.array_equal(a, b, equal_nan=True)
     assert np.any((one[6] == -1) & (s["nlist"] != -1))  # bonds broke
@@ -94,7 +94,16 @@ def test_same_bits(monkeypatch, form):
 
 @pytest.mark.parametrize("kind", ["euler", "euler_cromer"])
 def test_integrators(monkeypatch, kind):
-    one, _ = _run(monkeypatch, "volumes", kind, 2 ** 40, 50)
-    two, _ = _run(monkeypatch, "volumes", kind, 0, 50)
+    one, _ = _run(monkeypatch, "volumes", kind, False, 50)
+    two, _ = _run(monkeypatch, "volumes", kind, True, 50)
     for a, b in zip(one, two):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("width,bonds,expected", [
+    (32, 149_999, False), (32, 150_000, True), (33, 1, True),
+    (128, 6_818, True), (8, 1000, False), (256, 2 ** 30, False)])
+def test_rule(width, bonds, expected):
+    import torch
+    from probabilistic_peridynamics_gb300.pairs import worthwhile
+    assert worthwhile(1000, width, bonds, torch.device("cuda:0")) is expected
