@@ -741,13 +741,14 @@ int pp_rollout_forward(const pp_fused_args* args, const pp_pairs* pairs, const p
 /* The reverse of the rollout, its states recomputed segment by segment with
  * args->critical_stretch (infinite: frozen breaks).  args->nlist (=
  * adjoint->nlist) holds the bond set of the current step: scratch when
- * r->break_step is given, else the unbroken list.  lam0 = dL/du_steps; the
- * result dL/du_0 ends in lam0 or lam1 (steps even or odd).  grad_pair
+ * r->break_step is given, else the unbroken list.  grad_u (nnodes, 3) =
+ * dL/du_steps; mu0 and mu1 (nnodes, 4), 32-byte aligned: scratch.  grad_pair
  * (npairs, 2), 16-byte aligned, is added to; pp_pair_gradient writes it as
  * (nnodes, max_neigh). */
 int pp_rollout_backward(const pp_fused_args* args, const pp_pairs* pairs, const pp_rollout* r,
-                        const pp_adjoint_args* adjoint, const int32_t* nlist0, double* lam0,
-                        double* lam1, double* grad_pair, void* stream);
+                        const pp_adjoint_args* adjoint, const int32_t* nlist0,
+                        const double* grad_u, double* mu0, double* mu1, double* grad_pair,
+                        void* stream);
 int pp_pair_gradient(const pp_pairs* pairs, int64_t nslots, const double* grad_pair, double* grad,
                      void* stream);
 

@@ -254,7 +254,8 @@ SIGNATURES = {
     "pp_rollout_backward": (
         ctypes.c_int, [ctypes.POINTER(FusedArgs), ctypes.POINTER(Pairs),
                        ctypes.POINTER(RolloutArgs),
-                       ctypes.POINTER(AdjointArgs), _vp, _vp, _vp, _vp, _vp]),
+                       ctypes.POINTER(AdjointArgs), _vp, _vp, _vp, _vp, _vp,
+                       _vp]),
     "pp_pair_gradient": (ctypes.c_int, [ctypes.POINTER(Pairs), _i64, _vp, _vp,
                                         _vp]),
     "pp_fused_run_static": (

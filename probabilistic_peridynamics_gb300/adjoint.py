@@ -176,9 +176,9 @@ class AdjointProblem:
         broke = bool((breaks != INT32_MAX).any().item())
         # the bond set of the current step: without breaks, all of them
         nl = self.nlist0.clone()
-        lam = [grad_u.detach().to(torch.float64).reshape(-1, 3).clone(
-            memory_format=torch.contiguous_format)]
-        lam.append(torch.empty_like(lam[0]))
+        grad_u = grad_u.detach().to(torch.float64).reshape(-1, 3).contiguous()
+        mu = torch.empty((2, self.nnodes, 4), dtype=torch.float64,
+                         device=k.device)
         states = torch.empty((max(min(every, steps) - 1, 1), self.nnodes, 3),
                              dtype=torch.float64, device=k.device)
         grad_pair = torch.zeros((max(self.pairs.struct.npairs, 1), 2),
@@ -187,14 +187,14 @@ class AdjointProblem:
                              device=k.device)
         a = self._fused_args(nl, k, float("inf"))
         # (the states of each step are set by the call)
-        a.u[0], a.u[1] = states.data_ptr(), lam[1].data_ptr()
+        a.u[0], a.u[1] = states.data_ptr(), mu.data_ptr()
         r = self._rollout_args(steps, every, checkpoints,
                                breaks if broke else None, states)
         pairs = ctypes.byref(self.pairs.struct)
         check(lib().pp_rollout_backward(
             ctypes.byref(a), pairs, ctypes.byref(r),
             ctypes.byref(self._adjoint_args(nl, k)), _p(self.nlist0),
-            _p(lam[0]), _p(lam[1]), _p(grad_pair), self._stream),
+            _p(grad_u), _p(mu[0]), _p(mu[1]), _p(grad_pair), self._stream),
             "pp_rollout_backward")
         check(lib().pp_pair_gradient(pairs, grad_k.numel(), _p(grad_pair),
                                      _p(grad_k), self._stream),

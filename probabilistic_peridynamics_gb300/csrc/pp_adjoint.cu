@@ -114,15 +114,15 @@ __global__ void __launch_bounds__(kWarps * 32)
 
 constexpr int kPairThreads = 128;
 
-// What a bond's reverse step needs of its geometry: s, 1/|xi|, 1/|p|.
+// What a bond's reverse step needs of its geometry: s and 1/|p|.
 struct AdjointBond {
-    uint64_t s, inv_xi, inv_y;
+    uint64_t s, inv_y;
 };
 
 static __device__ __noinline__ AdjointBond adjoint_bond_any(double sq, double xi) {
     using exact64::double_bits;
     const double y = sqrt(sq);
-    return {double_bits((y - xi) / xi), double_bits(1.0 / xi), double_bits(1.0 / y)};
+    return {double_bits((y - xi) / xi), double_bits(1.0 / y)};
 }
 
 // On the integer pipe (pp_exact64.cuh) within the limits of f64_stretch.
@@ -130,36 +130,66 @@ __device__ __forceinline__ AdjointBond adjoint_bond(double sq, double xi) {
     using namespace exact64;
     const uint64_t sb = double_bits(sq), lb = double_bits(xi);
     constexpr uint64_t kOne = 0x3FF0000000000000ull;
-    AdjointBond r{0, 0, 0};
+    AdjointBond r{0, 0};
     bool ok = positive_in(sb, 1023 - 400, 1023 + 400) && positive_in(lb, 1023 - 200, 1023 + 200);
     if (ok) {
-        const Divisor y = sqrt_rn(sb), x = divisor(lb);
-        ok = relative_difference(y, x, r.s);
+        const Divisor y = sqrt_rn(sb);
+        ok = relative_difference(y, divisor(lb), r.s);
         r.inv_y = div_bits(kOne, y);
-        r.inv_xi = div_bits(kOne, x);
     }
     if (!ok) r = adjoint_bond_any(sq, xi);
     return r;
 }
 
-__device__ __forceinline__ d3 free_part(const double* __restrict__ lam,
-                                        const int32_t* __restrict__ bc, int64_t o) {
-    return d3{bc[o] ? 0.0 : lam[o], bc[o + 1] ? 0.0 : lam[o + 1], bc[o + 2] ? 0.0 : lam[o + 2]};
+// x, or zero where `off`: selected as integers (a selected double takes a
+// slot of the binary64 pipe).
+__device__ __forceinline__ double zero_if(bool off, const double* x) {
+    const long long bits = *reinterpret_cast<const long long*>(x);
+    return __longlong_as_double(off ? 0ll : bits);
+}
+
+// What the reverse step reads of a node, 32 bytes: lambda on the free DOFs
+// (zero on the others) and the volume.
+struct NodeMu {
+    d3 mu;
+    double vol;
+};
+
+__device__ __forceinline__ NodeMu load_mu(const double* __restrict__ mu, int64_t i) {
+    NodeMu r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(r.mu.x), "=d"(r.mu.y), "=d"(r.mu.z), "=d"(r.vol)
+        : "l"(mu + 4 * i));
+    return r;
+}
+
+__global__ void k_adjoint_pack(const double* __restrict__ grad_u, const int32_t* __restrict__ bc,
+                               const double* __restrict__ vols, int nnodes,
+                               double* __restrict__ mu) {
+    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (g >= 4 * (int64_t)nnodes) return;
+    const int64_t i = g >> 2, o = 3 * i + (g & 3);
+    mu[g] = (g & 3) == 3 ? vols[i] : zero_if(bc[o] != 0, grad_u + o);
 }
 
 __device__ __forceinline__ double dot(const d3& a, const d3& b) {
     return __fma_rn(a.x, b.x, __fma_rn(a.y, b.y, a.z * b.z));
 }
 
-// One thread per pair.  Bound by the binary64 pipe: about 45 operations a bond
-// (fused multiply-adds, root and reciprocals on the integer pipe) instead of
-// some 130 from each end, six of them divisions and two square roots.  A pass of the
-// 12,500-node rollout (500 steps forward, recomputed and reversed): 353 ms
-// with k_fused_f64 of the time and k_adjoint_backward, 228 ms after the forward steps'
-// arithmetic moved, 86 ms with both on pairs.
+// One thread per pair.  s/|p| = 1/|xi| - 1/|p|, so with c = s/|p|
+//   G v = c v + (p.v) p / |p|^3,   v = k_(j,m) vol_m mu_j - k_(m,j) vol_j mu_m
+// and both p.v and the gradients follow from p.mu_m and p.mu_j.  Bound by the
+// binary64 pipe: 39 operations a bond (fused multiply-adds; root and
+// quotients on the integer pipe) instead of some 130 from each end, six of
+// them divisions and two square roots.  What it gathers of a node is one load
+// (NodeMu) besides u.  A pass of the 12,500-node rollout (500 steps forward,
+// recomputed and reversed): 353 ms with k_fused_f64 of the time and
+// k_adjoint_backward, 228 ms after the forward steps' arithmetic moved, 79 ms
+// with both on pairs, 73 ms with this algebra, the nodes' records and
+// tree_block_f64 (this kernel 46 -> 43 us, k_adjoint_nodes 19 -> 17).
 __global__ void __launch_bounds__(kPairThreads)
     k_adjoint_pairs(pp_adjoint_args a, pp_pairs pr, int shift, const double* __restrict__ u,
-                    const double* __restrict__ lam_next, double* __restrict__ grad_pair) {
+                    const double* __restrict__ mu, double* __restrict__ grad_pair) {
     __shared__ double s_one;
     if (threadIdx.x == 0) s_one = 1.0;
     __syncthreads();
@@ -170,58 +200,80 @@ __global__ void __launch_bounds__(kPairThreads)
     const bool live_g = a.nlist[gh.x] != -1, live_h = a.nlist[gh.y] != -1;
     if (!live_g && !live_h) return;
     const int m = gh.x >> shift, j = gh.y >> shift;
-    const int64_t om = 3 * (int64_t)m, oj = 3 * (int64_t)j;
+    const int64_t om = 3 * (int64_t)m;
+    const NodeMu nm = load_mu(mu, m), nj = load_mu(mu, j);
+    const d3 mu_m = nm.mu, mu_j = nj.mu;
+    const double vol_m = nm.vol, vol_j = nj.vol;
+    const double kj = zero_if(!live_h, a.stiffness + gh.y);
+    const double km = zero_if(!live_g, a.stiffness + gh.x);
+    double2* const g = reinterpret_cast<double2*>(grad_pair) + q;
+    const double2 old = *g;
     const d3 p = f64_deformed(op, u, j, d3{u[om], u[om + 1], u[om + 2]},
                               pair_reference(pr, q));
     const AdjointBond bond = adjoint_bond(dot(p, p), pr.length[q]);
-    const double s = __longlong_as_double(bond.s);
     const double inv_y = __longlong_as_double(bond.inv_y);
-    const d3 h{p.x * inv_y, p.y * inv_y, p.z * inv_y};
-    const d3 mu_m = free_part(lam_next, a.bc_types, om), mu_j = free_part(lam_next, a.bc_types, oj);
-    const double vol_m = a.vols[m], vol_j = a.vols[j];
-    // v = k_(j,m) vol_m mu_j - k_(m,j) vol_j mu_m over the live directions
-    const double cj = live_h ? a.stiffness[gh.y] * vol_m : 0.0;
-    const double cm = live_g ? a.stiffness[gh.x] * vol_j : 0.0;
-    const d3 v{__fma_rn(cj, mu_j.x, -(cm * mu_m.x)), __fma_rn(cj, mu_j.y, -(cm * mu_m.y)),
-               __fma_rn(cj, mu_j.z, -(cm * mu_m.z))};
-    // G v = (s/|p|) v + (1/|xi| - s/|p|) (h.v) h
-    const double c2 = s * inv_y;
-    const double c1 = (__longlong_as_double(bond.inv_xi) - c2) * dot(h, v);
-    store_record(pr.force + 4 * q, d3{__fma_rn(c2, v.x, c1 * h.x), __fma_rn(c2, v.y, c1 * h.y),
-                                      __fma_rn(c2, v.z, c1 * h.z)});
-    // dL/dk += dt vol s (mu . h), h reversed for the second slot
-    const double t = a.dt * s;
-    double2* g = reinterpret_cast<double2*>(grad_pair) + q;
-    double2 sum = *g;
-    if (live_g) sum.x = __fma_rn(t * vol_j, dot(mu_m, h), sum.x);
-    if (live_h) sum.y = __fma_rn(-(t * vol_m), dot(mu_j, h), sum.y);
-    *g = sum;
+    const double c = __longlong_as_double(bond.s) * inv_y;
+    const double pm = dot(p, mu_m), pj = dot(p, mu_j);
+    const double cj = kj * vol_m, cm = -(km * vol_j);
+    const double e = __fma_rn(cj, pj, cm * pm) * inv_y * inv_y * inv_y;
+    const double wj = c * cj, wm = c * cm;
+    store_record(pr.force + 4 * q, d3{__fma_rn(wj, mu_j.x, __fma_rn(wm, mu_m.x, e * p.x)),
+                                      __fma_rn(wj, mu_j.y, __fma_rn(wm, mu_m.y, e * p.y)),
+                                      __fma_rn(wj, mu_j.z, __fma_rn(wm, mu_m.z, e * p.z))});
+    // dL/dk += dt vol s (mu . p)/|p|, p reversed for the second slot; a
+    // broken direction's stays as it is
+    const double t = a.dt * c;
+    const double gx = __fma_rn(t * vol_j, pm, old.x);
+    const double gy = __fma_rn(-(t * vol_m), pj, old.y);
+    longlong2 sum;
+    sum.x = live_g ? __double_as_longlong(gx) : __double_as_longlong(old.x);
+    sum.y = live_h ? __double_as_longlong(gy) : __double_as_longlong(old.y);
+    *reinterpret_cast<longlong2*>(g) = sum;
 }
 
-// lam = mu + dt (sum of the node's records), one warp per node.
+// lam = mu + dt (sum of the node's records), one warp per node; kept on the
+// free DOFs, with the volume.  A lane's slots go in batches of B, the loads of
+// a batch in flight together.
+template <int B>
 __global__ void __launch_bounds__(kWarps * 32)
-    k_adjoint_nodes(pp_adjoint_args a, pp_pairs pr, const double* __restrict__ lam_next,
-                    double* __restrict__ lam) {
-    const int lane = threadIdx.x & 31;
+    k_adjoint_nodes(pp_adjoint_args a, pp_pairs pr, const double* __restrict__ mu_next,
+                    double* __restrict__ mu) {
+    __shared__ double s_one, s_sum[3 * kWarps], s_part[3 * 32 * kWarps];
+    if (threadIdx.x == 0) s_one = 1.0;
+    __syncthreads();
+    const F64Ops op(&s_one);
     const int m = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    if (m >= a.nnodes) return;  // warp-uniform
     const int64_t row = (int64_t)m * a.max_neigh;
     d3 v = d3_zero();
-    for (int s = lane; s < a.max_neigh; s += 32) {
-        const int sp = pr.slot_pair[row + s];
-        if (a.nlist[row + s] == -1 || sp == -1) continue;
-        v = d3_add(v, signed_record(pr.force + 4 * (int64_t)(sp & 0x7FFFFFFF), sp));
+    for (int s0 = m < a.nnodes ? threadIdx.x & 31 : a.max_neigh; s0 < a.max_neigh;
+         s0 += 32 * B) {
+        int sp[B], j[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            sp[b] = pr.slot_pair[row + s0 + 32 * b];
+            j[b] = a.nlist[row + s0 + 32 * b];
+        }
+        d3 w[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            if (j[b] == -1) sp[b] = -1;
+            w[b] = signed_record(pr.force + 4 * (int64_t)(sp[b] & 0x7FFFFFFF), sp[b]);
+        }
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            v = d3{op.add(v.x, w[b].x), op.add(v.y, w[b].y), op.add(v.z, w[b].z)};
     }
-    // packed as in tree_reduce_f64: x on lane 0, z on 8, y on 16
-    const bool up16 = lane & 16, up8 = lane & 8;
-    const double xy = (up16 ? v.y : v.x) + shfl_xor(up16 ? v.x : v.y, 16);
-    const double z = v.z + shfl_xor(v.z, 16);
-    double t = (up8 ? z : xy) + shfl_xor(up8 ? xy : z, 8);
-    for (int off = 4; off >= 1; off >>= 1) t += shfl_xor(t, off);
-    if (lane == 0 || lane == 8 || lane == 16) {
-        const int64_t o = 3 * (int64_t)m + (lane == 0 ? 0 : (lane == 8 ? 2 : 1));
-        lam[o] = __fma_rn(a.dt, t, a.bc_types[o] ? 0.0 : lam_next[o]);
-    }
+    tree_block_put(s_part, v);
+    __syncthreads();
+    const int t = (threadIdx.x - 96 * blockIdx.x) & (kWarps * 32 - 1);
+    if (t < 96) tree_block_f64(op, t, s_part, s_sum);
+    __syncthreads();
+    const int64_t g = 4 * (int64_t)blockIdx.x * kWarps + threadIdx.x;
+    if (threadIdx.x >= 4 * kWarps || g >= 4 * (int64_t)a.nnodes) return;
+    const int node = threadIdx.x >> 2, comp = threadIdx.x & 3;
+    const double lam = __fma_rn(a.dt, s_sum[comp < 3 ? 3 * node + comp : 0], mu_next[g]);
+    const bool off = comp == 3 || a.bc_types[3 * (g >> 2) + comp] != 0;
+    mu[g] = off ? mu_next[g] : lam;  // (zero and the volume stay)
 }
 
 // The gradient of every slot from those kept per pair (zero elsewhere).
@@ -305,12 +357,15 @@ namespace pp {
 namespace {
 
 int adjoint_pair_step(const pp_adjoint_args& a, const pp_pairs& pr, const double* u,
-                      const double* lam_next, double* lam, double* grad_pair, cudaStream_t st) {
+                      const double* mu_next, double* mu, double* grad_pair, cudaStream_t st) {
     const int shift = 31 - __builtin_clz((unsigned)a.max_neigh);
     if (pr.npairs > 0)
         k_adjoint_pairs<<<(unsigned)((pr.npairs + kPairThreads - 1) / kPairThreads), kPairThreads,
-                          0, st>>>(a, pr, shift, u, lam_next, grad_pair);
-    k_adjoint_nodes<<<(a.nnodes + kWarps - 1) / kWarps, kWarps * 32, 0, st>>>(a, pr, lam_next, lam);
+                          0, st>>>(a, pr, shift, u, mu_next, grad_pair);
+    const auto nodes = a.max_neigh >= 128  ? k_adjoint_nodes<4>
+                       : a.max_neigh >= 64 ? k_adjoint_nodes<2>
+                                           : k_adjoint_nodes<1>;
+    nodes<<<(a.nnodes + kWarps - 1) / kWarps, kWarps * 32, 0, st>>>(a, pr, mu_next, mu);
     return launch_status();
 }
 
@@ -353,14 +408,15 @@ extern "C" int pp_rollout_forward(const pp_fused_args* args, const pp_pairs* pai
 
 extern "C" int pp_rollout_backward(const pp_fused_args* args, const pp_pairs* pairs,
                                    const pp_rollout* r, const pp_adjoint_args* adjoint,
-                                   const int32_t* nlist0, double* lam0, double* lam1,
-                                   double* grad_pair, void* stream) {
+                                   const int32_t* nlist0, const double* grad_u, double* mu0,
+                                   double* mu1, double* grad_pair, void* stream) {
     int v = check_rollout(args, pairs, r);
     if (v != PP_SUCCESS || args->nnodes == 0) return v;
     if (!adjoint || adjoint->nnodes != args->nnodes || adjoint->max_neigh != args->max_neigh ||
         adjoint->nlist != args->nlist || !adjoint->r0 || !adjoint->vols || !adjoint->bc_types ||
-        !adjoint->stiffness || !lam0 || !lam1 || lam0 == lam1 || !grad_pair ||
+        !adjoint->stiffness || !grad_u || !mu0 || !mu1 || mu0 == mu1 || !grad_pair ||
         (r->every > 1 && !r->states) || (r->break_step && !nlist0) ||
+        ((reinterpret_cast<uintptr_t>(mu0) | reinterpret_cast<uintptr_t>(mu1)) & 31u) ||
         (reinterpret_cast<uintptr_t>(grad_pair) & 15u))
         return PP_ERROR_INVALID_VALUE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -369,7 +425,10 @@ extern "C" int pp_rollout_backward(const pp_fused_args* args, const pp_pairs* pa
     pp_fused_args a = *args;
     pp_pairs pr = *pairs;
     pr.break_step = nullptr;
-    double* lam[2] = {lam0, lam1};
+    double* mu[2] = {mu0, mu1};
+    k_adjoint_pack<<<(unsigned)((4 * (int64_t)a.nnodes + 255) / 256), 256, 0, st>>>(
+        grad_u, adjoint->bc_types, adjoint->vols, a.nnodes, mu0);
+    if ((v = launch_status()) != PP_SUCCESS) return v;
     int p = 0;
     // the bond set in force during step t
     auto bonds = [&](int t) {
@@ -390,8 +449,7 @@ extern "C" int pp_rollout_backward(const pp_fused_args* args, const pp_pairs* pa
         }
         for (int t = t1 - 1; t >= t0; --t) {
             if ((v = bonds(t)) != PP_SUCCESS) return v;
-            if ((v = adjoint_pair_step(*adjoint, pr, state(t), lam[p], lam[p ^ 1], grad_pair,
-                                       st)) != PP_SUCCESS)
+            if ((v = adjoint_pair_step(*adjoint, pr, state(t), mu[p], mu[p ^ 1], grad_pair, st)) != PP_SUCCESS)
                 return v;
             p ^= 1;
         }

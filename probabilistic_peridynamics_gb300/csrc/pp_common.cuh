@@ -81,10 +81,9 @@ constexpr size_t tree_stack_bytes(int threads) {
 }
 
 // Reduce per-slot binary64 vectors of one node held by one warp, in the
-// work-group tree order.  SL = slots per lane = max(1, L/32).  `slot(k)`
-// returns the contribution of slot k and is called exactly once for every
-// slot < L (and for no other), on all lanes together.  Returns the sum's x on
-// lane 0, z on lane 8 and y on lane 16.
+// work-group tree order, down to one vector a lane.  SL = slots per lane =
+// max(1, L/32).  `slot(k)` returns the contribution of slot k and is called
+// exactly once for every slot < L (and for no other), on all lanes together.
 //
 // A lane's slots come in bit-reversed order, so that the tree's first
 // log2(SL) steps need one pending sum per level: `stack` (shared memory, 3
@@ -93,16 +92,12 @@ constexpr size_t tree_stack_bytes(int threads) {
 // of the slot's code, whatever SL), and the additions are branched around,
 // not predicated: a predicated DADD still takes the binary64 pipe's time.
 //
-// The last five steps pack the components: a step's lower half computes one
-// component while the upper half computes another (addition commutes, so the
-// sums are the tree's own): 6 additions a warp instead of 15.
-//
 // B slots of a lane are asked for together: slot(k, v) fills v[b] for slots
 // k[b], b < B (a power of two up to SL).  One at a time keeps the registers of
 // long slot code down; four at once keep four loads in flight.
 template <int SL, int B, class SlotFn>
-__device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, int L, double* stack,
-                                                  int stride, SlotFn&& slot) {
+__device__ __forceinline__ d3 tree_lane_f64(const F64Ops& op, int lane, int L, double* stack,
+                                            int stride, SlotFn&& slot) {
     static_assert(SL % B == 0, "whole batches");
     d3 v = d3_zero();
     if constexpr (SL == 1) {
@@ -111,11 +106,6 @@ __device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, in
             d3 one[1];
             slot(k, one);
             v = one[0];
-        }
-        if (L < 32) {
-            for (int off = L >> 1; off >= 1; off >>= 1) v = d3_add(v, d3_shfl_down(v, off));
-            const double y = __shfl_sync(kFull, v.y, 0), z = __shfl_sync(kFull, v.z, 0);
-            return lane == 0 ? v.x : (lane == 8 ? z : y);
         }
     } else {
         auto add = [&](const d3& a, const d3& b) {
@@ -152,6 +142,20 @@ __device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, in
             }
         }
     }
+    return v;
+}
+
+// The last steps of the tree, over the lanes of a node's warp.  Returns the
+// sum's x on lane 0, z on lane 8 and y on lane 16.  Rows of 32 slots or more
+// pack the components: a step's lower half computes one component while the
+// upper half computes another (addition commutes, so the sums are the tree's
+// own): 6 additions a warp instead of 15.
+__device__ __forceinline__ double tree_warp_f64(const F64Ops& op, int lane, int L, d3 v) {
+    if (L < 32) {
+        for (int off = L >> 1; off >= 1; off >>= 1) v = d3_add(v, d3_shfl_down(v, off));
+        const double y = __shfl_sync(kFull, v.y, 0), z = __shfl_sync(kFull, v.z, 0);
+        return lane == 0 ? v.x : (lane == 8 ? z : y);
+    }
     const bool up16 = lane & 16, up8 = lane & 8;
     const double xy = op.add(up16 ? v.y : v.x, shfl_xor(up16 ? v.x : v.y, 16));
     const double z = op.add(v.z, shfl_xor(v.z, 16));
@@ -159,6 +163,47 @@ __device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, in
 #pragma unroll
     for (int off = 4; off >= 1; off >>= 1) t = op.add(t, shfl_xor(t, off));
     return t;
+}
+
+// Both parts of the tree.
+template <int SL, int B, class SlotFn>
+__device__ __forceinline__ double tree_reduce_f64(const F64Ops& op, int lane, int L, double* stack,
+                                                  int stride, SlotFn&& slot) {
+    return tree_warp_f64(op, lane, L, tree_lane_f64<SL, B>(op, lane, L, stack, stride, slot));
+}
+
+// tree_warp_f64 for the eight nodes of a block of eight warps together (rows
+// of 32 slots or more): 24 sums of 32 words, four lanes a sum, on three of
+// the warps.  27 additions a block instead of 48 (the step on pairs: 400,000
+// nodes in rows of 128 slots 0.981 ms with, 1.020 without; 200,000 nodes in
+// rows of 32 0.201 and 0.223; 2,000 nodes 9.7 us and 10.4).  The words lie
+// where the lanes' stacks are: room of their own leaves less L1 to the records
+// (0.307 against 0.297 ms where every direction has a record).
+__device__ __forceinline__ void tree_block_put(double* stack, const d3& v) {
+    double* p = stack + threadIdx.x;
+    p[0] = v.x;
+    p[256] = v.y;
+    p[512] = v.z;
+}
+
+// After a barrier, by threads t = 0 .. 95: sum[3 node + component].  A sum's
+// lane takes words a + 4 (k ^ node): the steps of the tree pair k with k ^ 4,
+// k ^ 2 and k ^ 1, whatever k counts from, and eight sums read all banks.
+__device__ __forceinline__ void tree_block_f64(const F64Ops& op, int t, const double* stack,
+                                               double* sum) {
+    const int node = (t >> 2) & 7;
+    const double* p = stack + (t >> 5) * 256 + node * 32 + (t & 3);
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = p[4 * (k ^ node)];
+#pragma unroll
+    for (int s = 4; s >= 1; s >>= 1) {
+#pragma unroll
+        for (int k = 0; k < s; ++k) v[k] = op.add(v[k], v[k + s]);
+    }
+    double w = op.add(v[0], shfl_xor(v[0], 2));
+    w = op.add(w, shfl_xor(w, 1));
+    if ((t & 3) == 0) sum[3 * node + (t >> 5)] = w;
 }
 
 // ------------------------------------------------------------ double-float

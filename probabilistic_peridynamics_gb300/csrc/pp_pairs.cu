@@ -12,8 +12,8 @@
 //  k_pair_nodes  one warp per node: the records of its slots summed in the
 //                work-group tree order (pp_common.cuh), then the node update.
 //
-// Both kernels are bound by the binary64 pipe (87 and 89 % busy on the plate of
-// 400,000 nodes in rows of 128 slots: 0.63 + 0.39 ms), so halving the bond
+// Both kernels are bound by the binary64 pipe (88 and 85 % busy on the plate of
+// 400,000 nodes in rows of 128 slots: 0.63 + 0.34 ms), so halving the bond
 // work (1.95 ms in one kernel) outweighs writing and gathering the records (32 bytes
 // a pair written, 32 gathered per slot).  What that pipe does not have to do is
 // kept off it: roots and quotients (pp_exact64.cuh), the reference vectors
@@ -261,7 +261,8 @@ __global__ void __launch_bounds__(kPairThreads, 8)
 // Latency-bound until four slots' loads are in flight and the node updates'
 // inputs are staged (0.56 -> 0.43 ms); then 32 registers, so that 64 warps
 // are resident (0.39 ms; rows of 256 slots hold more and do better with 48:
-// 0.354 against 0.369 ms a step at 68,000 nodes).
+// 0.354 against 0.369 ms a step at 68,000 nodes), then the last steps of a
+// block's sums together (tree_block_f64: 0.34 ms).
 template <int SL, bool SYM>
 __global__ void __launch_bounds__(kRowWarps * 32, SL <= 4 ? 8 : 6)
     k_pair_nodes(pp_fused_args a, pp_pairs pr, int parity, Launch l) {
@@ -275,12 +276,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, SL <= 4 ? 8 : 6)
     const int warp = threadIdx.x >> 5;
     const int node0 = blockIdx.x * kRowWarps;
     const int i = node0 + warp;
+    const bool whole = SL > 1 || a.max_neigh == 32;  // a word for every lane
     f64_stage_nodes(a, parity, node0, kRowWarps, stage);
     if (i < a.nnodes) {  // warp-uniform
         const int64_t row = (int64_t)i * a.max_neigh;
         int intact = 0;
         constexpr int kBatch = SL < 4 ? SL : 4;
-        const double f = tree_reduce_f64<SL, kBatch>(
+        const d3 part = tree_lane_f64<SL, kBatch>(
             op, lane, a.max_neigh, s_stack + threadIdx.x, kRowWarps * 32,
             [&](const int(&k)[kBatch], d3(&v)[kBatch]) {
                 // all indices of a batch, then all its records
@@ -299,12 +301,21 @@ __global__ void __launch_bounds__(kRowWarps * 32, SL <= 4 ? 8 : 6)
                 }
             });
         const int count = __reduce_add_sync(kFull, intact);
-        if (lane == 0) {
-            stage.sum[3 * warp] = f;
-            stage.count[warp] = count;
+        if (lane == 0) stage.count[warp] = count;
+        if (whole) {
+            tree_block_put(s_stack, part);
+        } else {
+            const double f = tree_warp_f64(op, lane, a.max_neigh, part);
+            if (lane == 0) stage.sum[3 * warp] = f;
+            if (lane == 16) stage.sum[3 * warp + 1] = f;
+            if (lane == 8) stage.sum[3 * warp + 2] = f;
         }
-        if (lane == 16) stage.sum[3 * warp + 1] = f;
-        if (lane == 8) stage.sum[3 * warp + 2] = f;
+    }
+    if (whole) {
+        __syncthreads();
+        // on other warps from block to block (0.981 against 1.013 ms)
+        const int t = (threadIdx.x - 96 * blockIdx.x) & (kRowWarps * 32 - 1);
+        if (t < 96) tree_block_f64(op, t, s_stack, stage.sum);
     }
     f64_node_phase(a, parity, step_mags(l), node0, kRowWarps, stage);
 }
@@ -321,7 +332,7 @@ template <int SL>
 void launch_nodes(const pp_fused_args& a, const pp_pairs& pr, int parity, const Launch& l,
                   cudaStream_t st) {
     const unsigned grid = (unsigned)((a.nnodes + kRowWarps - 1) / kRowWarps);
-    constexpr size_t dyn = tree_stack_bytes<SL>(kRowWarps * 32);
+    constexpr size_t dyn = tree_stack_bytes<SL == 1 ? 2 : SL>(kRowWarps * 32);
     if (pr.symmetric)
         k_pair_nodes<SL, true><<<grid, kRowWarps * 32, dyn, st>>>(a, pr, parity, l);
     else

@@ -13,16 +13,16 @@ from ._lib import check, lib
 
 #: Rows of at most this many slots are one load a lane in the one-kernel step,
 #: which a second kernel beats only from ``MIN_BONDS`` directed bonds (one step,
-#: one kernel against pairs: 23,000 bonds 5.4 against 6.8 us, 56,000 bonds 6.7
-#: against 7.7, 97,000 bonds 8.0 against 8.6, 173,000 bonds 13.4 against 10.8,
-#: 3.5M bonds 268 against 223).  Wider rows are a serial loop over their slots
-#: there, so pairs are faster at every size (rows of 64: 39,000 bonds 7.9
-#: against 6.9 us, 94,000 bonds 10.2 against 8.7; rows of 128: 6,800 bonds 10.1
-#: against 7.4, 167,000 bonds 14.6 against 10.5, 2.9M bonds 139 against 80,
-#: 42.7M bonds 1,950 against 1,010; rows of 256: 121,000 bonds 18.8 against
-#: 10.5, 3.6M bonds 153 against 95).
+#: one kernel against pairs: 23,000 bonds 5.5 against 6.4 us, 81,000 bonds 7.4
+#: against 7.7, 97,000 bonds 8.0 against 7.8, 111,000 bonds 12.7 against 8.3,
+#: 6.1M bonds 354 against 199).  Wider rows are a serial loop over their slots
+#: there, so pairs are faster at every size (rows of 64: 39,000 bonds 8.0
+#: against 6.8 us, 94,000 bonds 9.9 against 8.0; rows of 128: 6,800 bonds 10.2
+#: against 7.0, 167,000 bonds 14.8 against 9.7, 2.9M bonds 139 against 77,
+#: 42.7M bonds 1,958 against 971; rows of 256: 121,000 bonds 18.6 against
+#: 10.1, 3.6M bonds 153 against 93).
 NARROW = 32
-MIN_BONDS = 150_000
+MIN_BONDS = 100_000
 
 _MAX_SLOTS = 2 ** 31 - 1
 _MAX_PAIRS = 2 ** 30 - 1

@@ -19,7 +19,7 @@ pytestmark = [pytest.mark.gpu,
 
 FORMS = ["plain", "unsorted", "holes", "one_sided", "twice", "own", "volumes",
          "corrections", "symmetric_corrections", "types", "types_corrections",
-         "instances", "wide", "narrow"]
+         "instances", "wide", "narrow", "row32", "row64"]
 
 
 def _model(form, kind):
@@ -42,8 +42,9 @@ def _model(form, kind):
             nl[i, s["family"][i]] = i if form == "own" else nl[i, 1]
     elif form == "wide":
         nl = np.concatenate([nl, np.full((n, 512 - w), -1, nl.dtype)], axis=1)
-    elif form == "narrow":
-        nl = np.ascontiguousarray(nl[:, :8])
+    elif form in ("narrow", "row32", "row64"):
+        nl = np.ascontiguousarray(
+            nl[:, :{"narrow": 8, "row32": 32, "row64": 64}[form]])
     n, w = nl.shape
     if form == "volumes":
         s["volume"] = s["volume"] * rng.uniform(0.5, 1.5, n)
@@ -101,7 +102,7 @@ def test_integrators(monkeypatch, kind):
 
 
 @pytest.mark.parametrize("width,bonds,expected", [
-    (32, 149_999, False), (32, 150_000, True), (33, 1, True),
+    (32, 99_999, False), (32, 100_000, True), (33, 1, True),
     (128, 6_818, True), (8, 1000, False), (256, 2 ** 30, False)])
 def test_rule(width, bonds, expected):
     import torch
