@@ -109,3 +109,17 @@ def test_edge_cases():
     fam, nl, width = _gpu(np.ones((50, 3)), 0.0)
     assert np.all(fam == 49) and width == 64
     assert np.array_equal(nl[3, :49], np.delete(np.arange(50), 3))
+
+
+@pytest.mark.parametrize("cells", [(1, 1, 1), (1, 1, 2), (1, 3, 1), (2, 1, 3),
+                                   (4, 2, 2), (2, 3, 5)])
+def test_few_cells_in_a_direction(cells):
+    """Grids whose columns of cells are cut by the faces."""
+    rng = np.random.default_rng(6)
+    coords = rng.uniform(0.0, 1.0, (400, 3)) * (np.array(cells) * 0.999)
+    fam, nl, _ = _gpu(coords, 1.0)
+    hit = _brute(coords, 1.0)
+    assert np.array_equal(fam, hit.sum(1))
+    for i in range(len(coords)):
+        assert np.array_equal(nl[i, :fam[i]], np.flatnonzero(hit[i]))
+        assert np.all(nl[i, fam[i]:] == -1)
