@@ -73,3 +73,48 @@ def test_same_bits(form):
     for a, b in zip(one, two):
         assert np.array_equal(a, b, equal_nan=True)
     assert int(setup["n_neigh"].sum() - two[4].sum()) > 50  # bonds broke
+
+
+@pytest.mark.parametrize("form", ["ascending", "shuffled", "one_sided",
+                                  "twice", "twice_one_sided", "own", "range"])
+def test_symmetry_count(form):
+    """Entries whose row does not hold them back as often, against a count on
+    the host."""
+    import torch
+    from probabilistic_peridynamics_gb300._lib import check, lib
+    s = _lattice(7, 6, 4, 3.1)
+    rng = np.random.default_rng(1)
+    nl, n_neigh = s["nlist"].copy(), s["family"].copy()
+    n = nl.shape[0]
+    nl = np.concatenate([nl, np.zeros((n, 3), nl.dtype)], axis=1)
+
+    def add(i, j):
+        nl[i, n_neigh[i]] = j
+        n_neigh[i] += 1
+    if form == "shuffled":
+        for i in range(n):
+            rng.shuffle(nl[i, :n_neigh[i]])
+    elif form == "one_sided":
+        n_neigh[::5] -= 1
+    elif form.startswith("twice"):
+        for i in range(0, n, 7):
+            j = nl[i, 2]
+            add(i, j)
+            if form == "twice":
+                add(j, i)
+    elif form == "own":
+        for i in range(0, n, 3):
+            add(i, i)
+    elif form == "range":
+        nl[3, 1], nl[8, 0] = n, -2
+    rows = [nl[i, :n_neigh[i]].tolist() for i in range(n)]
+    want = sum(j < 0 or j >= n or rows[i].count(j) != rows[j].count(i)
+               for i in range(n) for j in rows[i])
+    dev = [torch.from_numpy(np.ascontiguousarray(x, dtype=np.int32)).cuda()
+           for x in (nl, n_neigh)]
+    bad = torch.empty(1, dtype=torch.int32, device="cuda")
+    check(lib().pp_cy_check_symmetric(
+        dev[0].data_ptr(), dev[1].data_ptr(), n, nl.shape[1], bad.data_ptr(),
+        torch.cuda.current_stream().cuda_stream), "pp_cy_check_symmetric")
+    assert int(bad.item()) == want
+    assert (want == 0) == (form in ("ascending", "shuffled", "twice", "own"))
