@@ -186,7 +186,8 @@ __device__ __forceinline__ double dot(const d3& a, const d3& b) {
 // recomputed and reversed): 353 ms with k_fused_f64 of the time and
 // k_adjoint_backward, 228 ms after the forward steps' arithmetic moved, 79 ms
 // with both on pairs, 73 ms with this algebra, the nodes' records and
-// tree_block_f64 (this kernel 46 -> 43 us, k_adjoint_nodes 19 -> 17).
+// tree_block_f64 (this kernel 46 -> 43 us, k_adjoint_nodes 19 -> 17), 68 ms
+// with the forward kernels launched ahead (pp_pairs.cu).
 __global__ void __launch_bounds__(kPairThreads)
     k_adjoint_pairs(pp_adjoint_args a, pp_pairs pr, int shift, const double* __restrict__ u,
                     const double* __restrict__ mu, double* __restrict__ grad_pair) {

@@ -60,6 +60,35 @@ struct F64Ops {
     __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nzero); }
 };
 
+// Programmatic dependent launch: a kernel launched by launch_dependent may be
+// brought up before the one before it in the stream has ended; each of its
+// threads calls grid_wait() before it reads or writes memory, which returns
+// when that one is complete and its writes are visible.  Not for kernels with
+// `const __restrict__` parameters or read-only loads at addresses known before
+// the wait, which the compiler may move ahead of it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The next kernel may be brought up when every block has come here or ended.
+__device__ __forceinline__ void grid_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... Params, class... Args>
+void launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem,
+                      cudaStream_t st, const Args&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, Params(args)...);  // (launch_status() has its error)
+}
+
 __device__ __forceinline__ double shfl_xor(double v, int off) {
     return __shfl_xor_sync(kFull, v, off);
 }

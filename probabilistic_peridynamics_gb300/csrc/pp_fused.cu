@@ -20,8 +20,8 @@ namespace pp {
 namespace {
 
 // Four warps a block: 24 warps per SM at 80 registers, and a block's node
-// updates wait for four warps only (400,000-node plate, rows of 128 slots:
-// 2.69 ms against 2.72 with eight; 2000 nodes 19.8 against 20.6 us).
+// updates wait for four warps only (measured with more work on the FP64 pipe:
+// 2,000 nodes 19.8 against 20.6 us with eight).
 constexpr int kDefaultWarps = 4;
 
 // One warp per node for the bond phase; the node updates of the block's
@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parit
     const int warp = threadIdx.x >> 5;
     const int node0 = blockIdx.x * wpb;
     const int i = node0 + warp;
+    grid_wait();
     f64_stage_nodes(a, parity, node0, wpb, stage);
     const StepMags m = step_mags(l);
     const double* __restrict__ u = a.u[parity];
@@ -136,9 +137,10 @@ namespace {
 template <int SL, bool CORR, bool TYPES>
 void launch_f64_variant(const pp_fused_args& a, int parity, const Launch& l, cudaStream_t st) {
     const int wpb = a.nodes_per_block > 0 ? a.nodes_per_block : kDefaultWarps;
-    const dim3 grid((a.nnodes + wpb - 1) / wpb), block(32 * wpb);
-    k_fused_f64<SL, CORR, TYPES>
-        <<<grid, block, tree_stack_bytes<SL>(32 * wpb), st>>>(a, parity, l);
+    const unsigned grid = (unsigned)((a.nnodes + wpb - 1) / wpb), block = 32u * wpb;
+    // (2,116 nodes in rows of 32 slots: 6.5 us a step, 6.7 launched after the last)
+    launch_dependent(k_fused_f64<SL, CORR, TYPES>, grid, block, tree_stack_bytes<SL>(block), st, a,
+                     parity, l);
 }
 
 template <int SL>

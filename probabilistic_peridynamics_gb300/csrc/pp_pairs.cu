@@ -31,6 +31,14 @@ namespace {
 
 constexpr int kRowWarps = 8;
 constexpr int kPairThreads = 128;
+// The step's kernels are launched ahead of their predecessor's end
+// (pp_common.cuh: 2,000 nodes 9.2 us a step against 9.7, 800 nodes in rows of 256
+// slots 9.7 against 10.1).  From so many pairs on they also let the next one in
+// before their last stores (42.7M bonds 0.944 against 0.968 ms, 6.1M bonds in rows
+// of 32 slots 0.179 against 0.194, 1.0M bonds 30.1 against 30.4 us); with fewer its
+// waiting blocks crowd the SMs (470,000 bonds 16.3 against 15.1 us, 36,500 bonds
+// 10.6 against 6.9).
+constexpr int kReleasePairs = 400'000;
 constexpr int kSingle = -2;    // build: owner of a pair of one side
 constexpr int kPartner = -3;   // build: the pair's other slot owns it
 
@@ -196,6 +204,7 @@ __global__ void __launch_bounds__(kPairThreads, 8)
     __syncthreads();
     const F64Ops op(&s_one);
     const int64_t p = blockIdx.x * (int64_t)kPairThreads + threadIdx.x;
+    grid_wait();
     if (p >= pr.npairs) return;
     const int2 gh = __ldg(reinterpret_cast<const int2*>(pr.slots) + p);
     const int jg = a.nlist[gh.x];
@@ -221,6 +230,7 @@ __global__ void __launch_bounds__(kPairThreads, 8)
     const d3 ui{b.u[oi], b.u[oi + 1], b.u[oi + 2]};
     const d3 xe = f64_deformed(op, b.u, j, ui, pair_reference(pr, p));
     const F64Stretch st = f64_stretch<false>(op, xe, pr.length[p]);
+    if (pr.npairs >= kReleasePairs) grid_release();
     bool live_g = jg != -1, live_h = jh != -1;
     const double s = __longlong_as_double(st.s);
     if constexpr (SYM) {
@@ -276,6 +286,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, SL <= 4 ? 8 : 6)
     const int warp = threadIdx.x >> 5;
     const int node0 = blockIdx.x * kRowWarps;
     const int i = node0 + warp;
+    grid_wait();
     const bool whole = SL > 1 || a.max_neigh == 32;  // a word for every lane
     f64_stage_nodes(a, parity, node0, kRowWarps, stage);
     if (i < a.nnodes) {  // warp-uniform
@@ -317,6 +328,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, SL <= 4 ? 8 : 6)
         const int t = (threadIdx.x - 96 * blockIdx.x) & (kRowWarps * 32 - 1);
         if (t < 96) tree_block_f64(op, t, s_stack, stage.sum);
     }
+    if (pr.npairs >= kReleasePairs) grid_release();
     f64_node_phase(a, parity, step_mags(l), node0, kRowWarps, stage);
 }
 
@@ -325,7 +337,8 @@ void launch_bonds(const pp_fused_args& a, const pp_pairs& pr, int parity, cudaSt
     const int shift = 31 - __builtin_clz((unsigned)a.max_neigh);
     const int64_t grid = (pr.npairs + kPairThreads - 1) / kPairThreads;
     if (grid > 0)
-        k_pair_bonds<CORR, TYPES, SYM><<<(unsigned)grid, kPairThreads, 0, st>>>(a, pr, parity, shift);
+        launch_dependent(k_pair_bonds<CORR, TYPES, SYM>, (unsigned)grid, kPairThreads, 0, st, a, pr,
+                         parity, shift);
 }
 
 template <int SL>
@@ -334,9 +347,9 @@ void launch_nodes(const pp_fused_args& a, const pp_pairs& pr, int parity, const 
     const unsigned grid = (unsigned)((a.nnodes + kRowWarps - 1) / kRowWarps);
     constexpr size_t dyn = tree_stack_bytes<SL == 1 ? 2 : SL>(kRowWarps * 32);
     if (pr.symmetric)
-        k_pair_nodes<SL, true><<<grid, kRowWarps * 32, dyn, st>>>(a, pr, parity, l);
+        launch_dependent(k_pair_nodes<SL, true>, grid, kRowWarps * 32, dyn, st, a, pr, parity, l);
     else
-        k_pair_nodes<SL, false><<<grid, kRowWarps * 32, dyn, st>>>(a, pr, parity, l);
+        launch_dependent(k_pair_nodes<SL, false>, grid, kRowWarps * 32, dyn, st, a, pr, parity, l);
 }
 
 }  // namespace

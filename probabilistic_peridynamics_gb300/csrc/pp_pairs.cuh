@@ -18,13 +18,14 @@ __device__ __forceinline__ d3 pair_reference(const pp_pairs& pr, int64_t p) {
     return d3{pr.vector[p], pr.vector[pr.npairs + p], pr.vector[2 * pr.npairs + p]};
 }
 
-// The record at p where `live`, else +0 (without a branch around the load).
+// The record at p where `live`, else +0 (without a branch around the load).  Not
+// a read-only load: a dependent launch may begin before the records are written.
 __device__ __forceinline__ d3 load_record_if(const double* p, bool live) {
     d3 v{0.0, 0.0, 0.0};
     [[maybe_unused]] double w = 0.0;
     asm("{\n\t.reg .pred live;\n\t"
         "setp.ne.s32 live, %5, 0;\n\t"
-        "@live ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];\n\t}"
+        "@live ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n\t}"
         : "+d"(v.x), "+d"(v.y), "+d"(v.z), "+d"(w)
         : "l"(p), "r"((int)live));
     return v;

@@ -19,7 +19,7 @@ from ._lib import check, lib
 #: there, so pairs are faster at every size (rows of 64: 39,000 bonds 8.0
 #: against 6.8 us, 94,000 bonds 9.9 against 8.0; rows of 128: 6,800 bonds 10.2
 #: against 7.0, 167,000 bonds 14.8 against 9.7, 2.9M bonds 139 against 77,
-#: 42.7M bonds 1,958 against 971; rows of 256: 121,000 bonds 18.6 against
+#: 42.7M bonds 1,958 against 947; rows of 256: 121,000 bonds 18.6 against
 #: 10.1, 3.6M bonds 153 against 93).
 NARROW = 32
 MIN_BONDS = 100_000

@@ -19,13 +19,14 @@ pytestmark = [pytest.mark.gpu,
 
 FORMS = ["plain", "unsorted", "holes", "one_sided", "twice", "own", "volumes",
          "corrections", "symmetric_corrections", "types", "types_corrections",
-         "instances", "wide", "narrow", "row32", "row64"]
+         "instances", "wide", "narrow", "row32", "row64", "large"]
 
 
 def _model(form, kind):
     """(setup, keyword arguments of run_integrator) of one form."""
     rng = np.random.default_rng(3)
-    s = breaking_setup(kind)
+    # "large": enough pairs for kernels that let the next one in early
+    s = breaking_setup(kind, *((62, 51, 4) if form == "large" else ()))
     n, w = s["nlist"].shape
     nl = s["nlist"].copy()
     more = {}
@@ -81,6 +82,8 @@ def _run(monkeypatch, form, kind, pairs, steps):
     out = run_integrator(integ, s, steps, 3e-3 * np.arange(1, steps + 1),
                          force_mags=np.zeros(steps), use_run=True, **more)
     assert (integ._pairs is not None) == pairs
+    if pairs and form == "large":
+        assert integ._pairs.struct.npairs > 400_000
     return out, s
 
 
