@@ -13,14 +13,14 @@ from ._lib import check, lib
 
 #: Rows of at most this many slots are one load a lane in the one-kernel step,
 #: which a second kernel beats only from ``MIN_BONDS`` directed bonds (one step,
-#: one kernel against pairs: 23,000 bonds 5.5 against 6.4 us, 81,000 bonds 7.4
-#: against 7.7, 97,000 bonds 8.0 against 7.8, 111,000 bonds 12.7 against 8.3,
-#: 6.1M bonds 354 against 199).  Wider rows are a serial loop over their slots
-#: there, so pairs are faster at every size (rows of 64: 39,000 bonds 8.0
-#: against 6.8 us, 94,000 bonds 9.9 against 8.0; rows of 128: 6,800 bonds 10.2
-#: against 7.0, 167,000 bonds 14.8 against 9.7, 2.9M bonds 139 against 77,
-#: 42.7M bonds 1,958 against 947; rows of 256: 121,000 bonds 18.6 against
-#: 10.1, 3.6M bonds 153 against 93).
+#: one kernel against pairs: 23,000 bonds 5.2 against 6.0 us, 81,000 bonds 7.1
+#: against 7.3, 97,000 bonds 7.7 against 7.4, 111,000 bonds 12.3 against 7.8,
+#: 6.1M bonds 352 against 182).  Wider rows are a serial loop over their slots
+#: there, so pairs are faster at every size (rows of 64: 39,000 bonds 7.7
+#: against 6.4 us, 94,000 bonds 9.6 against 7.6; rows of 128: 6,800 bonds 9.8
+#: against 6.8, 167,000 bonds 14.5 against 9.3, 2.9M bonds 139 against 76,
+#: 42.7M bonds 1,959 against 954; rows of 256: 121,000 bonds 18.5 against
+#: 9.7, 3.6M bonds 153 against 93).
 NARROW = 32
 MIN_BONDS = 100_000
 
