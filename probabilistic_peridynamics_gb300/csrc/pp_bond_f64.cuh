@@ -37,12 +37,7 @@ struct F64Bond {
     int nregimes;
 };
 
-// Stretch and direction cosines of one bond: s = (y - xi) / xi, q = xe / y.
-// Kept as bits: where two paths join, the compiler merges doubles with an
-// instruction of the binary64 pipe each.
-struct F64Stretch {
-    uint64_t s, qx, qy, qz;
-};
+using F64Stretch = exact64::Stretch;
 
 // By the binary64 pipe's own operations: any inputs.
 static __device__ __noinline__ void f64_stretch_any(double x, double y, double z, double xi,
@@ -55,39 +50,17 @@ static __device__ __noinline__ void f64_stretch_any(double x, double y, double z
     out->qz = double_bits(ddiv(z, len));
 }
 
-// The same values by pp_exact64.cuh, which needs no binary64 instruction for
-// the root, the difference and the four quotients: ~140 clocks a warp and
-// slot of the integer and FP32 pipes instead of ~720 of the binary64 pipe,
-// which the other operations of the slot keep busy.  It takes lengths within
-// 2^+-200 (squares 2^+-400) that differ by less than a factor of two, and
-// components that are zero or above 2^-700, so that no intermediate is
-// subnormal or overflows; everything else (NaN and infinities among it)
-// goes to f64_stretch_any.
+// The same values by pp_exact64.cuh where it takes the operands: ~140 clocks a
+// warp and slot of the integer and FP32 pipes instead of ~720 of the binary64
+// pipe, which the other operations of the slot keep busy.
 //
 // kIntSquares: the three squares on the integer pipe too.  The one-kernel
 // steps, with 23 binary64 operations a slot, gain by it (rows of 128 slots 2.00 ->
 // 1.87, of 32 slots 0.38 -> 0.35 ms); the pair step, with 16, does not.
 template <bool kIntSquares>
 __device__ __forceinline__ F64Stretch f64_stretch(const F64Ops& op, const d3& xe, double xi) {
-    using namespace exact64;
-    const uint64_t xb = double_bits(xe.x), yb = double_bits(xe.y), zb = double_bits(xe.z);
-    const uint64_t lb = double_bits(xi);
     F64Stretch r{0, 0, 0, 0};
-    bool ok = positive_in(lb, 1023 - 200, 1023 + 200) && zero_or_above(xb, 1023 - 500) &&
-              zero_or_above(yb, 1023 - 500) && zero_or_above(zb, 1023 - 500);
-    if (ok) {
-        const double x2 = kIntSquares ? bits_double(square_bits(xb)) : op.mul(xe.x, xe.x);
-        const double y2 = kIntSquares ? bits_double(square_bits(yb)) : op.mul(xe.y, xe.y);
-        const double z2 = kIntSquares ? bits_double(square_bits(zb)) : op.mul(xe.z, xe.z);
-        const uint64_t sb = double_bits(op.add(op.add(x2, y2), z2));
-        ok = positive_in(sb, 1023 - 400, 1023 + 400);
-        const Divisor len = sqrt_rn(sb);
-        ok = relative_difference(len, divisor(lb), r.s) && ok;
-        r.qx = div_bits(xb, len);
-        r.qy = div_bits(yb, len);
-        r.qz = div_bits(zb, len);
-    }
-    if (!ok) {
+    if (!exact64::stretch_in_range<kIntSquares>(op, xe.x, xe.y, xe.z, xi, r)) {
         F64Stretch t;
         f64_stretch_any(xe.x, xe.y, xe.z, xi, &t);
         r = t;

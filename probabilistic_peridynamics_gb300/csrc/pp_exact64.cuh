@@ -283,7 +283,9 @@ PP_HD uint64_t div_bits(uint64_t a, const Divisor& d) {
     return is_zero(a) ? a : bits;
 }
 
-// bits of a a (+0 for a zero).
+// bits of a a (+0 for a zero).  A nonzero a is within 2^+-500, so that the
+// square is normal and its exponent stays inside its field: beyond, an infinity
+// or a NaN among it, the result is some other finite number.
 PP_HD uint64_t square_bits(uint64_t a) {
     const Num q = square_rn(unpack(a));
     return is_zero(a) ? 0 : pack(q.m, q.e);
@@ -319,14 +321,53 @@ PP_HD bool relative_difference(const Divisor& y, const Divisor& x, uint64_t& bit
     return (uint32_t)(de + 1) <= 2u && (m >> 53) == 0;
 }
 
-// Zero, or a number whose exponent field is at least lo.
-PP_HD bool zero_or_above(uint64_t bits, uint32_t lo) {
-    return ((uint32_t)(bits >> 32) << 1) >= (lo << 21) || is_zero(bits);
+// Zero, or a number of either sign whose exponent field is lo .. hi (hi - lo
+// below 1023); neither an infinity nor a NaN while hi is below 2047.
+PP_HD bool zero_or_in(uint64_t bits, uint32_t lo, uint32_t hi) {
+    return ((uint32_t)(bits >> 32) << 1) - (lo << 21) < ((hi + 1 - lo) << 21) || is_zero(bits);
 }
 
 // Is `bits` a positive number of exponent field lo .. hi (0 < lo)?
 PP_HD bool positive_in(uint64_t bits, uint32_t lo, uint32_t hi) {
     return (uint32_t)(bits >> 52) - lo <= hi - lo;
+}
+
+// Stretch and direction cosines of a bond, s = (y - xi) / xi and q = p / y with
+// y = |p|.  Kept as bits: where two paths join, the compiler merges doubles with
+// an instruction of the binary64 pipe each.
+struct Stretch {
+    uint64_t s, qx, qy, qz;
+};
+
+// The stretch of the bond with deformed vector (x, y, z) and reference length xi,
+// without a binary64 operation for the root, the difference and the four
+// quotients; op adds (and multiplies, without kIntSquares).  True when the
+// operands are in the range of these: lengths within 2^+-200 (squares 2^+-400)
+// that differ by less than a factor of two, and components that are zero or within
+// 2^-500 .. 2^201, so that no intermediate is subnormal or overflows.  Else r is
+// left to the caller (NaN and infinities among it).  The upper limit of the
+// components has to be tested before kIntSquares squares them: the sum of wrapped
+// squares can be in range.
+template <bool kIntSquares, class Ops>
+PP_HD bool stretch_in_range(const Ops& op, double x, double y, double z, double xi, Stretch& r) {
+    constexpr uint32_t kLo = 1023 - 500, kHi = 1023 + 200;
+    const uint64_t xb = double_bits(x), yb = double_bits(y), zb = double_bits(z);
+    const uint64_t lb = double_bits(xi);
+    bool ok = positive_in(lb, 1023 - 200, 1023 + 200) && zero_or_in(xb, kLo, kHi) &&
+              zero_or_in(yb, kLo, kHi) && zero_or_in(zb, kLo, kHi);
+    if (ok) {
+        const double x2 = kIntSquares ? bits_double(square_bits(xb)) : op.mul(x, x);
+        const double y2 = kIntSquares ? bits_double(square_bits(yb)) : op.mul(y, y);
+        const double z2 = kIntSquares ? bits_double(square_bits(zb)) : op.mul(z, z);
+        const uint64_t sb = double_bits(op.add(op.add(x2, y2), z2));
+        ok = positive_in(sb, 1023 - 400, 1023 + 400);
+        const Divisor len = sqrt_rn(sb);
+        ok = relative_difference(len, divisor(lb), r.s) && ok;
+        r.qx = div_bits(xb, len);
+        r.qy = div_bits(yb, len);
+        r.qz = div_bits(zb, len);
+    }
+    return ok;
 }
 
 }  // namespace exact64
