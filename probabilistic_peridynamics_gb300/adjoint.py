@@ -25,6 +25,7 @@ frozen in the backward pass: the loss is piecewise constant in the critical
 stretch, whose gradient is therefore zero.
 """
 import ctypes
+import threading
 
 import numpy as np
 
@@ -96,6 +97,9 @@ class AdjointProblem:
                                         _p(self.bond_length), self._stream),
                   "pp_bond_lengths")
             self.pairs = self._make_pairs()
+        # The pair list's force records pass from one kernel to the next, so
+        # the rollouts of several threads are queued one after the other.
+        self._queueing = threading.Lock()
 
     @property
     def _stream(self):
@@ -165,9 +169,10 @@ class AdjointProblem:
         a = self._fused_args(nl, k, critical_stretch)
         a.u[0], a.u[1] = u[0].data_ptr(), u[1].data_ptr()
         r = self._rollout_args(steps, every, checkpoints, breaks)
-        check(lib().pp_rollout_forward(
-            ctypes.byref(a), ctypes.byref(self.pairs.struct),
-            ctypes.byref(r), self._stream), "pp_rollout_forward")
+        with self._queueing:
+            check(lib().pp_rollout_forward(
+                ctypes.byref(a), ctypes.byref(self.pairs.struct),
+                ctypes.byref(r), self._stream), "pp_rollout_forward")
         return u[steps & 1], checkpoints, breaks
 
     def run_backward(self, grad_u, k, steps, every, checkpoints, breaks):
@@ -191,11 +196,12 @@ class AdjointProblem:
         r = self._rollout_args(steps, every, checkpoints,
                                breaks if broke else None, states)
         pairs = ctypes.byref(self.pairs.struct)
-        check(lib().pp_rollout_backward(
-            ctypes.byref(a), pairs, ctypes.byref(r),
-            ctypes.byref(self._adjoint_args(nl, k)), _p(self.nlist0),
-            _p(grad_u), _p(mu[0]), _p(mu[1]), _p(grad_pair), self._stream),
-            "pp_rollout_backward")
+        with self._queueing:
+            check(lib().pp_rollout_backward(
+                ctypes.byref(a), pairs, ctypes.byref(r),
+                ctypes.byref(self._adjoint_args(nl, k)), _p(self.nlist0),
+                _p(grad_u), _p(mu[0]), _p(mu[1]), _p(grad_pair),
+                self._stream), "pp_rollout_backward")
         check(lib().pp_pair_gradient(pairs, grad_k.numel(), _p(grad_pair),
                                      _p(grad_k), self._stream),
               "pp_pair_gradient")
