@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256, 3) k_fused_f64(pp_fused_args a, int parit
     grid_wait();
     f64_stage_nodes(a, parity, node0, wpb, stage);
     const StepMags m = step_mags(l);
-    const double* __restrict__ u = a.u[parity];
+    const double* u = a.u[parity];
     if (i < a.nnodes) {  // warp-uniform
         const F64Bond b{a.r0,
                         u,

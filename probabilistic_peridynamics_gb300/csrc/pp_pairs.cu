@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kPairThreads, 8)
     const int64_t p = blockIdx.x * (int64_t)kPairThreads + threadIdx.x;
     grid_wait();
     if (p >= pr.npairs) return;
-    const int2 gh = __ldg(reinterpret_cast<const int2*>(pr.slots) + p);
+    const int2 gh = reinterpret_cast<const int2*>(pr.slots)[p];
     const int jg = a.nlist[gh.x];
     const int jh = gh.y >= 0 ? a.nlist[gh.y] : -1;
     if (jg == -1 && jh == -1) return;

@@ -56,9 +56,10 @@ def fits(nnodes, max_neigh, bonds, device):
 class DevicePairs:
     """Device arrays of one pair list, built from the neighbour list (and
     volumes and corrections) of ``fargs``; queued on ``stream`` (a handle,
-    torch's current stream), which the call waits for.  With ``two_sided``
-    each direction of a bond keeps a force of its own, whatever the volumes
-    and corrections."""
+    torch's current stream).  The call waits for the count of the pairs, and
+    for the rest only where the two directions of a bond may share a force.
+    With ``two_sided`` each direction keeps a force of its own, whatever the
+    volumes and corrections."""
 
     def __init__(self, fargs, device, stream, two_sided=False):
         import torch
