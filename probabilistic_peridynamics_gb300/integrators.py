@@ -936,11 +936,9 @@ class Euler(Integrator):
                     "pp_bond_lengths")
 
     def _make_step(self):
+        """The arrays of a step (its numbers are set at every step)."""
         a = _lib.CyStep()
         a.nnodes, a.width = self.nnodes, self._width
-        a.bond_stiffness = float(self.bond_stiffness)
-        a.critical_strain = float(self.critical_stretch)
-        a.dt = float(self.dt)
         a.coords, a.volume = _ptr(self._coords_d), _ptr(self._volume_d)
         a.force_bc_values = _ptr(self._fc_values_d)
         a.force_bc_types = _ptr(self._fc_types_d)
@@ -969,6 +967,9 @@ class Euler(Integrator):
         L = lib()
         if self._pairs is not None:
             a = self._step
+            a.bond_stiffness = float(self.bond_stiffness)
+            a.critical_strain = float(self.critical_stretch)
+            a.dt = float(self.dt)
             a.force_bc_scale = float(force_bc_magnitude)
             a.bc_scale = float(displacement_bc_magnitude)
             check(L.pp_cy_pair_step(ctypes.byref(a),
