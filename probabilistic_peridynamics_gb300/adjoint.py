@@ -25,6 +25,7 @@ frozen in the backward pass: the loss is piecewise constant in the critical
 stretch, whose gradient is therefore zero.
 """
 import ctypes
+import operator
 import threading
 
 import numpy as np
@@ -237,6 +238,19 @@ class AdjointProblem:
         return lam
 
 
+def _counts(steps, every):
+    """Steps and checkpoint interval as plain integers (of any integer type;
+    an interval beyond the rollout is one checkpoint), or None where a pair
+    list does not take them."""
+    try:
+        steps, every = operator.index(steps), operator.index(every)
+    except TypeError:
+        return None
+    if steps < 0 or every < 1:
+        return None
+    return steps, min(every, max(steps, 1))
+
+
 def _rollout_function():
     import torch
 
@@ -251,13 +265,12 @@ def _rollout_function():
             with problem.context.on_stream():
                 k = stiffness.detach().to(torch.float64).contiguous()
                 s0 = float(critical_stretch)
-                # (a pair list takes plain step counts)
+                counts = _counts(steps, checkpoint_every)
                 paired = (problem.pairs is not None
                           and k.shape == problem.nlist0.shape
-                          and isinstance(steps, int) and steps >= 0
-                          and isinstance(checkpoint_every, int)
-                          and checkpoint_every >= 1)
+                          and counts is not None)
                 if paired:
+                    steps, checkpoint_every = counts
                     u, checkpoints, breaks = problem.run_forward(
                         k, steps, checkpoint_every, s0)
                 else:

@@ -4,12 +4,19 @@ import contextlib
 import ctypes
 
 import numpy as np
+import torch
 
 from probabilistic_peridynamics_gb300 import _lib, adjoint, lattice
 
 
+class FakeStream:
+    def wait_stream(self, other):
+        pass
+
+
 class FakeContext:
     device = "cpu"
+    stream = FakeStream()
     stream_handle = ctypes.c_void_p(0)
 
     def on_stream(self):
@@ -25,6 +32,9 @@ def fake_problem(monkeypatch, steps=8, **calls):
             return calls.get(name, lambda *args: _lib.PP_SUCCESS)
 
     library = Library()
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda *_: FakeContext.stream)
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda *_: None)
     monkeypatch.setattr(adjoint, "lib", lambda: library)
     coords = lattice.lattice_coords(4, 3, 2, 1.0)
     family, nlist, _ = lattice.lattice_family(4, 3, 2, 2.015)
