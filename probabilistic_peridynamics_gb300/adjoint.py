@@ -146,8 +146,12 @@ class AdjointProblem:
                       states=None):
         r = _lib.RolloutArgs()
         r.steps, r.every = steps, every
-        self.mags = np.ascontiguousarray(self.mags)
-        r.mags = self.mags.ctypes.data
+        # (read while the call runs; a caller may have assigned magnitudes of
+        # another type: whatever gives a number at each step)
+        mags = (self.mags if isinstance(self.mags, np.ndarray)
+                else [float(self.mags[t]) for t in range(steps)])
+        r.host_mags = np.ascontiguousarray(mags, dtype=np.float64)
+        r.mags = r.host_mags.ctypes.data
         r.checkpoints = _p(checkpoints)
         r.states = _p(states)
         r.break_step = _p(break_step)
