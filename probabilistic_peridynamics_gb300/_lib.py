@@ -303,12 +303,24 @@ def lib():
 COPY_BYTES = 8 << 20
 
 
+def host_lib():
+    """The library for plain host work, which goes on without it: None where
+    it cannot be loaded."""
+    try:
+        return lib()
+    except (LibraryError, OSError, AttributeError):
+        return None
+
+
 def host_copy(a):
     """``a.copy()``, a large C-contiguous array on several threads."""
-    if a.nbytes < COPY_BYTES or not a.flags.c_contiguous:
+    large = (type(a) is np.ndarray and a.nbytes >= COPY_BYTES
+             and a.flags.c_contiguous and not a.dtype.hasobject)
+    library = host_lib() if large else None
+    if library is None:
         return a.copy()
-    out = np.empty_like(a, subok=False)
-    check(lib().pp_host_copy(out.ctypes.data, a.ctypes.data, a.nbytes),
+    out = np.empty_like(a)
+    check(library.pp_host_copy(out.ctypes.data, a.ctypes.data, a.nbytes),
           "pp_host_copy")
     return out
 

@@ -16,7 +16,7 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
-from ._lib import check, host_copy, lib
+from ._lib import check, host_copy, host_lib
 
 
 @dataclass
@@ -104,10 +104,13 @@ class Batch:
             part = array[a:b]
             if kind == "nlist":
                 w = self.instances[k].nlist.shape[1]
-                if (part.dtype == np.int32 and part.ndim == 2
-                        and part.flags.c_contiguous):
+                native = (part.dtype == np.int32 and part.ndim == 2
+                          and part.flags.c_contiguous and part.shape[1] >= w
+                          and part.shape[0] == b - a)
+                library = host_lib() if native else None
+                if library is not None:
                     local = np.empty((b - a, w), dtype=np.int64)
-                    check(lib().pp_host_local_rows(
+                    check(library.pp_host_local_rows(
                         part.ctypes.data, b - a, part.shape[1], w, a,
                         local.ctypes.data), "pp_host_local_rows")
                     part = local
