@@ -29,6 +29,7 @@ queued on the context's CUDA stream and is asynchronous until ``write``.
 """
 from abc import ABC, abstractmethod
 import ctypes
+import threading
 
 import numpy as np
 
@@ -106,6 +107,12 @@ def _ptr(t):
 _REGISTER_BYTES = 4 << 20
 
 
+#: Held while an upload has a caller's array page-locked: threads may upload the
+#: same array (models that share their points), and the first to end would
+#: unlock the pages under the others' copies.
+_uploading = threading.Lock()
+
+
 def _upload(array, dtype, device):
     """A device tensor of ``array`` as ``dtype``.  A large array is
     page-locked for the copy (see ``_CUDAIntegrator._put``): 205 MB take 2 ms
@@ -113,17 +120,20 @@ def _upload(array, dtype, device):
     import torch
     a = np.ascontiguousarray(array, dtype=dtype)
     src = torch.as_tensor(a)
-    if a.nbytes < _REGISTER_BYTES or src.is_pinned():
+    if a.nbytes < _REGISTER_BYTES:
         return src.to(device, non_blocking=False)
-    out = torch.empty(a.shape, dtype=src.dtype, device=device)
-    registered = lib().pp_host_register(a.ctypes.data,
-                                        a.nbytes) == _lib.PP_SUCCESS
-    try:
-        out.copy_(src)
-    finally:
-        if registered:
-            lib().pp_host_unregister(a.ctypes.data)
-    return out
+    with _uploading:
+        if not src.is_pinned():
+            out = torch.empty(a.shape, dtype=src.dtype, device=device)
+            registered = lib().pp_host_register(
+                a.ctypes.data, a.nbytes) == _lib.PP_SUCCESS
+            try:
+                out.copy_(src)
+            finally:
+                if registered:
+                    lib().pp_host_unregister(a.ctypes.data)
+            return out
+    return src.to(device, non_blocking=False)
 
 
 def _bounds(coords):
