@@ -112,9 +112,12 @@ class AdjointProblem:
         bonds = int(self.family.sum().item())
         if not fits(self.nnodes, self.max_neigh, bonds, self.context.device):
             return None
-        pairs = DevicePairs(self._fused_args(self.nlist0, None, float("inf")),
-                            self.context.device, self._stream, two_sided=True)
-        return pairs if 2 * pairs.struct.npairs == bonds else None
+        pairs = DevicePairs.build(
+            self._fused_args(self.nlist0, None, float("inf")),
+            self.context.device, self._stream, bonds, two_sided=True)
+        if pairs is None or 2 * pairs.struct.npairs != bonds:
+            return None
+        return pairs
 
     def _fused_args(self, nlist, k, critical_stretch):
         """Arguments of a binary64 Euler step (without its states)."""

@@ -442,21 +442,23 @@ class _CUDAIntegrator(Integrator):
             self._create_mixed_buffers()
         self.bond_length_d = None
         self._pairs = None
-        pairs = self.fused and self.precision == "float64" and worthwhile(
-            n, mn, int(np.sum(n_neigh)), self.context.device)
-        if self.fused and self.precision == "float64" and not pairs:
-            # |xi| per slot, read by the fused binary64 step instead of a
-            # square root per bond and step (the same binary64 value)
-            self.bond_length_d = torch.empty(
-                (n, self.max_neighbours), dtype=torch.float64,
-                device=self.context.device)
-            check(lib().pp_bond_lengths(
-                _ptr(self.r0_d), _ptr(self.nlist_d), n, self.max_neighbours,
-                _ptr(self.bond_length_d), self._stream), "pp_bond_lengths")
         self._fargs = self._make_fused_args() if self.fused else None
-        if pairs:
-            self._pairs = DevicePairs(self._fargs, self.context.device,
-                                      self._stream)
+        if self.fused and self.precision == "float64":
+            bonds = int(np.sum(n_neigh))
+            if worthwhile(n, mn, bonds, self.context.device):
+                self._pairs = DevicePairs.build(
+                    self._fargs, self.context.device, self._stream, bonds)
+            if self._pairs is None:
+                # |xi| per slot, read by the fused binary64 step instead of a
+                # square root per bond and step (the same binary64 value)
+                self.bond_length_d = torch.empty(
+                    (n, self.max_neighbours), dtype=torch.float64,
+                    device=self.context.device)
+                check(lib().pp_bond_lengths(
+                    _ptr(self.r0_d), _ptr(self.nlist_d), n,
+                    self.max_neighbours, _ptr(self.bond_length_d),
+                    self._stream), "pp_bond_lengths")
+                self._fargs.bond_length = _ptr(self.bond_length_d)
         if self.precision == "mixed":
             if self.tiled:
                 from .tiling import DeviceTiling

@@ -27,6 +27,8 @@ MIN_BONDS = 100_000
 _MAX_SLOTS = 2 ** 31 - 1
 _MAX_PAIRS = 2 ** 30 - 1
 _SMALL_BYTES = 2 ** 25
+#: Slots, length, vector and two records.
+_PAIR_BYTES = 8 + 8 + 24 + 64
 
 
 def worthwhile(nnodes, max_neigh, bonds, device):
@@ -37,37 +39,47 @@ def worthwhile(nnodes, max_neigh, bonds, device):
 
 
 def fits(nnodes, max_neigh, bonds, device):
-    """Do the indices and the memory of a pair list fit?  Its arrays (four
-    bytes a slot and up to 52 a bond) may take half of the device memory that
-    is free, and no more; of a small list that is not asked (it takes longer
-    than building the list)."""
-    import torch
+    """Do the indices and the memory of a pair list fit?  Its arrays take four
+    bytes a slot and up to 52 a bond listed from both ends."""
     slots = nnodes * max_neigh
-    if slots > _MAX_SLOTS or bonds > _MAX_PAIRS:
-        return False
-    if 4 * slots + 52 * bonds <= _SMALL_BYTES:
-        return True
-    free = (torch.cuda.mem_get_info(device)[0]
+    return (slots <= _MAX_SLOTS and bonds <= _MAX_PAIRS
+            and _room(4 * slots + 52 * bonds, device))
+
+
+def _room(size, device):
+    """May the pair list's arrays take so many bytes?  Half of the device memory
+    that is free, and no more; for a small list that is not asked (it takes
+    longer than building the list)."""
+    return size <= _SMALL_BYTES or size <= _free_bytes(device) // 2
+
+
+def _free_bytes(device):
+    import torch
+    return (torch.cuda.mem_get_info(device)[0]
             + torch.cuda.memory_reserved(device)
             - torch.cuda.memory_allocated(device))
-    return 4 * slots + 52 * bonds <= free // 2
 
 
 class DevicePairs:
-    """Device arrays of one pair list, built from the neighbour list (and
-    volumes and corrections) of ``fargs``; queued on ``stream`` (a handle,
-    torch's current stream).  The call waits for the count of the pairs, and
-    for the rest only where the two directions of a bond may share a force.
-    With ``two_sided`` each direction keeps a force of its own, whatever the
-    volumes and corrections."""
+    """Device arrays of one pair list (see :meth:`build`)."""
 
-    def __init__(self, fargs, device, stream, two_sided=False):
+    @classmethod
+    def build(cls, fargs, device, stream, bonds, two_sided=False):
+        """The pair list of the neighbour list (and volumes and corrections) of
+        ``fargs``, or None where its arrays do not fit: a bond listed from one
+        end only, or more than once, is a pair of its own, with up to twice
+        the memory that :func:`fits` expects of ``bonds``.  Queued on ``stream`` (a handle,
+        torch's current stream); the call waits for the count of the pairs,
+        and for the rest only where the two directions of a bond may share a
+        force.  With ``two_sided`` each direction keeps a force of its own,
+        whatever the volumes and corrections."""
         import torch
         n, width = int(fargs.nnodes), int(fargs.max_neigh)
 
         def empty(shape, dtype):
             return torch.empty(shape, dtype=dtype, device=device)
 
+        self = cls()
         args = ctypes.byref(fargs)
         self.slot_pair = empty((n, width), torch.int32)
         start = empty((n + 1,), torch.int32)
@@ -76,6 +88,9 @@ class DevicePairs:
                                   start.data_ptr(), scratch.data_ptr(),
                                   stream), "pp_pair_count")
         npairs = int(start[n].item())
+        if npairs > _MAX_PAIRS or (2 * npairs > bonds and not _room(
+                _PAIR_BYTES * npairs, device)):
+            return None
         self.slots = empty((max(npairs, 1), 2), torch.int32)
         self.length = empty((max(npairs, 1),), torch.float64)
         self.vector = empty((3, max(npairs, 1)), torch.float64)
@@ -92,6 +107,7 @@ class DevicePairs:
         self.force = empty((max(npairs, 1) * (1 if s.symmetric else 2), 4),
                            torch.float64)
         s.force = self.force.data_ptr()
+        return self
 
 
 class CyPairs:

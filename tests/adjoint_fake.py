@@ -41,9 +41,11 @@ def fake_problem(monkeypatch, steps=8, **calls):
     bonds = int(np.sum(family))
 
     class Pairs:
-        def __init__(self, *args, **kwargs):
-            self.struct = _lib.Pairs()
-            self.struct.npairs = bonds // 2
+        struct = _lib.Pairs(npairs=bonds // 2)
+
+        @classmethod
+        def build(cls, *args, **kwargs):
+            return cls()
 
     monkeypatch.setattr(adjoint, "DevicePairs", Pairs)
     bc_types, bc_values = lattice.face_bcs(coords, 0)
