@@ -442,10 +442,11 @@ class _CUDAIntegrator(Integrator):
             self._create_mixed_buffers()
         self.bond_length_d = None
         self._pairs = None
-        self._fargs = self._make_fused_args() if self.fused else None
+        self._fargs = None
         if self.fused and self.precision == "float64":
             bonds = int(np.sum(n_neigh))
             if worthwhile(n, mn, bonds, self.context.device):
+                self._fargs = self._make_fused_args()
                 self._pairs = DevicePairs.build(
                     self._fargs, self.context.device, self._stream, bonds)
             if self._pairs is None:
@@ -458,7 +459,8 @@ class _CUDAIntegrator(Integrator):
                     _ptr(self.r0_d), _ptr(self.nlist_d), n,
                     self.max_neighbours, _ptr(self.bond_length_d),
                     self._stream), "pp_bond_lengths")
-                self._fargs.bond_length = _ptr(self.bond_length_d)
+        if self.fused and self._pairs is None:
+            self._fargs = self._make_fused_args()
         if self.precision == "mixed":
             if self.tiled:
                 from .tiling import DeviceTiling
