@@ -7,6 +7,7 @@ never changes the simulation state.  Results are cached per process by a
 problem key.
 """
 import ctypes
+import time
 
 from . import _lib
 from ._lib import check, lib
@@ -107,17 +108,46 @@ def _time_layout(integ, tiled, warmup, reps):
     return results
 
 
-#: The tiled layout is taken when its step is this much faster: it is built
-#: anew at every create_buffers, and a near tie would not repay that (250,000
-#: irregular nodes: steps of 95 against 97 us, but 200 steps with their set-up
-#: 43.9 against 38.9 ms) and would be settled by the noise of the timings.
+#: A tiled step that is less than this much faster has to repay the tiling,
+#: which is built anew at every create_buffers (see :func:`choose`).
 _TILED_GAIN = 0.95
 
 
-def _choose(results):
-    """The fastest candidate, the tiled ones handicapped by _TILED_GAIN."""
-    return min(results, key=lambda c: results[c]
-               / (_TILED_GAIN if c.startswith("tiled/") else 1.0))
+def choose(results, setup_ms, steps=None):
+    """The fastest candidate; in a near tie of the layouts, the untiled one
+    unless the run repays the tiling.
+
+    ``setup_ms`` is the time of building the tiling and ``steps`` the length
+    of the run, None where it is not known.  250,000 irregular nodes, steps of
+    93 us tiled and 97 us untiled, set-up 1.4 ms: calls of 50 steps take 16.7
+    against 16.0 ms, of 200 30.4 against 30.3, of 2,000 184.7 against 185.9.
+    """
+    best = min(results, key=results.get)
+    untiled = [c for c in results if c.startswith("untiled/")]
+    if not best.startswith("tiled/") or not untiled or steps is None:
+        return best
+    other = min(untiled, key=results.get)
+    gain = results[other] - results[best]
+    if results[best] > _TILED_GAIN * results[other] and steps * gain < setup_ms:
+        return other
+    return best
+
+
+def _key(integ):
+    """What the timings of an integrator's step depend on."""
+    return ("mixed", integ.nnodes, integ.max_neighbours, integ._kind,
+            integ.stiffness_corrections_d is not None,
+            integ.bond_types_d is not None, integ.node_instance_d is not None,
+            integ.compensated, integ._may_tile)
+
+
+def wants_tiling(integ):
+    """Does an integrator that may be tiled need its tiling: to time it, or
+    because it is known to be the choice for its planned run?"""
+    if not integ.autotune or _key(integ) not in _cache:
+        return True
+    return choose(*_cache[_key(integ)],
+                  integ.planned_steps).startswith("tiled/")
 
 
 def _apply(integ, choice):
@@ -127,32 +157,41 @@ def _apply(integ, choice):
     integ._fargs.variant = int(variant)
 
 
+def _time_setup(integ):
+    """Milliseconds of building the integrator's tiling once more."""
+    from .tiling import DeviceTiling
+    stream = integ.context.stream
+    stream.synchronize()
+    start = time.perf_counter()
+    integ._build_tiling(DeviceTiling(*integ._order, integ.context.device))
+    stream.synchronize()
+    return 1e3 * (time.perf_counter() - start)
+
+
 def tune_mixed(integ, warmup=3, reps=10):
     """Pick the layout and tile shape of a mixed-precision integrator.
 
     Times every tile shape of the untiled kernel and, when the integrator
-    was set up tiled, of the tiled kernel, and keeps the fastest (the tiled
-    kernel where it is clearly faster): an integrator whose untiled kernel
-    wins drops its tiling.
+    was set up tiled, of the tiled kernel, and keeps the one :func:`choose`
+    takes for the integrator's planned run: an integrator whose untiled
+    kernel wins drops its tiling.
 
     :returns: dict ``"layout/variant"`` -> milliseconds per step.
     """
     import torch
-    fa = integ._fargs
-    tiled = integ.tiling is not None
-    key = ("mixed", fa.nnodes, fa.max_neigh, fa.integrator,
-           bool(fa.stiffness_corrections), bool(fa.bond_types),
-           bool(fa.node_instance), fa.flags, tiled)
-    if key in _cache:
-        _apply(integ, _cache[key][0])
-        return _cache[key][1]
+    key = _key(integ)
+    if key not in _cache:
+        tiled = integ.tiling is not None
+        with integ.context.on_stream():
+            results, setup_ms = {}, 0.0
+            if tiled:
+                results.update(_time_layout(integ, True, warmup, reps))
+            results.update(_time_layout(integ, False, warmup, reps))
+            if tiled:
+                setup_ms = _time_setup(integ)
+        _cache[key] = (results, setup_ms)
+        torch.cuda.empty_cache()
+    results, setup_ms = _cache[key]
     with integ.context.on_stream():
-        results = {}
-        if tiled:
-            results.update(_time_layout(integ, True, warmup, reps))
-        results.update(_time_layout(integ, False, warmup, reps))
-        best = _choose(results)
-        _apply(integ, best)
-    _cache[key] = (best, results)
-    torch.cuda.empty_cache()
+        _apply(integ, choose(results, setup_ms, integ.planned_steps))
     return results

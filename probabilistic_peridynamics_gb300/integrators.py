@@ -227,8 +227,12 @@ class _CUDAIntegrator(Integrator):
         self.autotune = bool(autotune)
         # mixed precision: gather neighbour records from shared memory on
         # the tiled layout (False: the untiled kernel, from L1/L2)
-        self.tiled = bool(tiled) and precision == "mixed"
+        self._may_tile = bool(tiled) and precision == "mixed"
+        self.tiled = self._may_tile  # the layout of the current buffers
         self.tiling = None
+        # steps of the run that the next create_buffers begins, where its
+        # caller knows them (Model.simulate does)
+        self.planned_steps = None
         self.tile_target = 125  # nodes per brick of the internal order
         self._order = None
         self.tuning = None
@@ -333,7 +337,7 @@ class _CUDAIntegrator(Integrator):
         self._torch = torch
         if self.precision == "mixed":
             self._coord_bounds = _bounds(self.coords) if self.nnodes else None
-        if self.tiled:
+        if self._may_tile:
             from .tiling import brick_order
             self._order = brick_order(
                 self.coords, None if self._instances is None
@@ -439,6 +443,9 @@ class _CUDAIntegrator(Integrator):
         self.damage_d = self._zeros((n,), torch.float64)
         self._parity = 0
         if self.precision == "mixed":
+            from .autotune import tune_mixed, wants_tiling
+            self.tiled = self._may_tile and wants_tiling(self)
+            self.tiling = None
             self._create_mixed_buffers()
         self.bond_length_d = None
         self._pairs = None
@@ -464,21 +471,24 @@ class _CUDAIntegrator(Integrator):
         if self.precision == "mixed":
             if self.tiled:
                 from .tiling import DeviceTiling
-                self.tiling = DeviceTiling(*self._order, self.context.device)
-                self.tiling.build(
-                    self._fargs, self._stream,
-                    corrections=self.stiffness_corrections_d is not None,
-                    types=self.bond_types_d is not None,
-                    instances=self.node_instance_d is not None)
+                self.tiling = self._build_tiling(
+                    DeviceTiling(*self._order, self.context.device))
                 # (tiles split to fit the halo capacity stay split)
                 self._order = (self._order[0], self.tiling.tile_start)
                 self._fargs.tiling = ctypes.addressof(self.tiling.struct)
             check(lib().pp_mixed_pack(ctypes.byref(self._fargs), 0,
                                       self._stream), "pp_mixed_pack")
             if self.autotune:
-                from .autotune import tune_mixed
                 self.tuning = tune_mixed(self)
+        self.planned_steps = None
         self._create_special_buffers()
+
+    def _build_tiling(self, tiling):
+        return tiling.build(
+            self._fargs, self._stream,
+            corrections=self.stiffness_corrections_d is not None,
+            types=self.bond_types_d is not None,
+            instances=self.node_instance_d is not None)
 
     def _drop_tiling(self):
         """Switch a mixed-precision integrator set up tiled to the untiled

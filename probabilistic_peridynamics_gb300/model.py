@@ -862,6 +862,8 @@ class Model(object):
                 'force': np.zeros(nwrites, dtype=np.float64),
                 'body_force': np.zeros(nwrites, dtype=np.float64),
                 'damage_sum': np.zeros(nwrites, dtype=np.float64)}
+        if hasattr(self.integrator, "planned_steps"):
+            self.integrator.planned_steps = steps
         self.integrator.create_buffers(
             nlist, n_neigh, bond_stiffness, critical_stretch, plus_cs, u, ud,
             udd, force, body_force, damage, regimes, nregimes, nbond_types)
