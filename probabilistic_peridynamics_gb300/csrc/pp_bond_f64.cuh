@@ -50,22 +50,24 @@ static __device__ __noinline__ void f64_stretch_any(double x, double y, double z
     out->qz = double_bits(ddiv(z, len));
 }
 
+struct F64StretchAny {
+    __device__ __forceinline__ void operator()(double x, double y, double z, double xi,
+                                               F64Stretch* out) const {
+        f64_stretch_any(x, y, z, xi, out);
+    }
+};
+
 // The same values by pp_exact64.cuh where it takes the operands: ~140 clocks a
 // warp and slot of the integer and FP32 pipes instead of ~720 of the binary64
 // pipe, which the other operations of the slot keep busy.
 //
 // kIntSquares: the three squares on the integer pipe too.  The one-kernel
-// steps, with 23 binary64 operations a slot, gain by it (rows of 128 slots 2.00 ->
-// 1.87, of 32 slots 0.38 -> 0.35 ms); the pair step, with 16, does not.
+// steps, with 23 binary64 operations a slot, gain by it (400,000 nodes in rows of
+// 128 slots: plain 2.51 -> 2.09 ms, fused 1.99 -> 1.97; 90,000 in rows of 32: 170 ->
+// 157 us, fused 165 -> 152); the pair step, with 16, does not.
 template <bool kIntSquares>
 __device__ __forceinline__ F64Stretch f64_stretch(const F64Ops& op, const d3& xe, double xi) {
-    F64Stretch r{0, 0, 0, 0};
-    if (!exact64::stretch_in_range<kIntSquares>(op, xe.x, xe.y, xe.z, xi, r)) {
-        F64Stretch t;
-        f64_stretch_any(xe.x, xe.y, xe.z, xi, &t);
-        r = t;
-    }
-    return r;
+    return exact64::stretch<kIntSquares>(op, xe, xi, F64StretchAny());
 }
 
 // |xi| from the squared length, correctly rounded.

@@ -1,10 +1,10 @@
 """The range of the integer route of the bond arithmetic, on the CPU.
 
-``stretch_in_range`` (``csrc/pp_exact64.cuh``, which also compiles for the
-host) says whether it computed a bond.  Whatever it takes must equal IEEE
-binary64 arithmetic bit for bit; components that are huge, infinite or NaN are
-not its to take, whatever stands beside them, with squares in integers and
-with squares by the caller's multiplication.
+``stretch`` (``csrc/pp_exact64.cuh``, which also compiles for the host) leaves
+to its caller's function what is outside its range.  Whatever it takes itself
+must equal IEEE binary64 arithmetic bit for bit; components that are huge,
+infinite or NaN are not its to take, whatever stands beside them, with squares
+in integers and with squares by the caller's multiplication.
 """
 import ctypes
 import itertools
@@ -24,14 +24,22 @@ struct Ops {
     double add(double a, double b) const { return a + b; }
     double mul(double a, double b) const { return a * b; }
 };
+struct Vec { double x, y, z; };
+struct Any {
+    int* taken;
+    void operator()(double, double, double, double, Stretch* r) const {
+        *taken = 0;
+        *r = Stretch{0, 0, 0, 0};
+    }
+};
 extern "C" void run(long n, int squares, const double* p, const double* xi,
                     double* out, int* taken) {
     for (long i = 0; i < n; ++i) {
-        Stretch r{0, 0, 0, 0};
-        const double *v = p + 3 * i;
-        taken[i] = squares
-            ? stretch_in_range<true>(Ops(), v[0], v[1], v[2], xi[i], r)
-            : stretch_in_range<false>(Ops(), v[0], v[1], v[2], xi[i], r);
+        const Vec v{p[3 * i], p[3 * i + 1], p[3 * i + 2]};
+        taken[i] = 1;
+        const Any any{taken + i};
+        const Stretch r = squares ? stretch<true>(Ops(), v, xi[i], any)
+                                  : stretch<false>(Ops(), v, xi[i], any);
         const uint64_t bits[4] = {r.s, r.qx, r.qy, r.qz};
         for (int k = 0; k < 4; ++k) out[4 * i + k] = bits_double(bits[k]);
     }
