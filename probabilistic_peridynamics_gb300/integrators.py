@@ -114,9 +114,15 @@ _uploading = threading.Lock()
 
 
 def _upload(array, dtype, device):
-    """A device tensor of ``array`` as ``dtype``.  A large array is
-    page-locked for the copy (see ``_CUDAIntegrator._put``): 205 MB take 2 ms
-    instead of 11."""
+    """A device tensor of ``array`` as ``dtype``.
+
+    A large array is page-locked for the copy (see ``_CUDAIntegrator._put``).
+    Most copies of unlocked memory are as fast (130 MB in use 0.8 ms, 1.2
+    locked; 68 MB of untouched zeros 3.6, 2.8 locked), but some take many
+    times as long (130 MB 7 to 20 ms): calls of 250,000 mixed-precision nodes
+    take 31.5 ms instead of 29.3 when only the arrays of 32 MB or more are
+    locked.
+    """
     import torch
     a = np.ascontiguousarray(array, dtype=dtype)
     src = torch.as_tensor(a)
