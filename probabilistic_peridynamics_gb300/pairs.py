@@ -48,15 +48,21 @@ def fits(nnodes, max_neigh, bonds, device):
 
 def _room(size, device):
     """May the pair list's arrays take so many bytes?  Half of the device memory
-    that is free, and no more; for a small list that is not asked (it takes
-    longer than building the list)."""
-    return size <= _SMALL_BYTES or size <= _free_bytes(device) // 2
+    that is free, and no more; for a small list that is not asked, and what
+    torch keeps for reuse is only where the rest does not do (the three
+    questions take as long as building the list)."""
+    return (size <= _SMALL_BYTES or 2 * size <= _free_bytes(device)
+            or 2 * size <= _free_bytes(device) + _cached_bytes(device))
 
 
 def _free_bytes(device):
     import torch
-    return (torch.cuda.mem_get_info(device)[0]
-            + torch.cuda.memory_reserved(device)
+    return torch.cuda.mem_get_info(device)[0]
+
+
+def _cached_bytes(device):
+    import torch
+    return (torch.cuda.memory_reserved(device)
             - torch.cuda.memory_allocated(device))
 
 
