@@ -35,7 +35,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import check, lib
-from .pairs import CyPairs, DevicePairs, fits, worthwhile
+from .pairs import CyPairs, DevicePairs, cy_worthwhile, worthwhile
 
 
 class ContextError(Exception):
@@ -458,7 +458,8 @@ class _CUDAIntegrator(Integrator):
         self._fargs = None
         if self.fused and self.precision == "float64":
             bonds = int(np.sum(n_neigh))
-            if worthwhile(n, mn, bonds, self.context.device):
+            if worthwhile(n, mn, bonds, self.context.device,
+                          self.planned_steps):
                 self._fargs = self._make_fused_args()
                 self._pairs = DevicePairs.build(
                     self._fargs, self.context.device, self._stream, bonds)
@@ -839,8 +840,8 @@ class Euler(Integrator):
         :arg float dt: The length of time (in seconds [s]) of one time-step.
         :arg device_context: Optional :class:`CUDAContext` for the kernels.
         :arg bool fused: True: each bond computed once over a list of pairs
-            (``pp_cy_pair_step``; where that does not fit,
-            ``pp_cy_break_and_force``); False: one kernel per Cython
+            (``pp_cy_pair_step``; where that does not fit or the run is too
+            short to repay the list, ``pp_cy_break_and_force``); False: one kernel per Cython
             function.  Same results.
         """
         if device_context is not None and not isinstance(device_context,
@@ -850,6 +851,9 @@ class Euler(Integrator):
         self.fused = bool(fused)
         # Not a device-layout integrator: Model builds the compact layout
         self.context = None
+        # steps of the run that the next create_buffers begins, where its
+        # caller knows them (Model.simulate does)
+        self.planned_steps = None
         self._device = device_context
         lib()  # fail loudly now if the CUDA library is missing
 
@@ -950,8 +954,11 @@ class Euler(Integrator):
                                          device=self.device_context.device)
             self._l0_d = None
             self._pairs = None
-            if self.fused and fits(n, width, int(np.sum(n_neigh)),
-                                   self.device_context.device):
+            pairs = self.fused and cy_worthwhile(
+                n, width, int(np.sum(n_neigh)), self.device_context.device,
+                self.planned_steps)
+            self.planned_steps = None
+            if pairs:
                 self._step = self._make_step()
                 self._pairs = CyPairs(self._step, self.device_context.device,
                                       self.device_context.stream_handle)

@@ -31,11 +31,31 @@ _SMALL_BYTES = 2 ** 25
 _PAIR_BYTES = 8 + 8 + 24 + 64
 
 
-def worthwhile(nnodes, max_neigh, bonds, device):
+def worthwhile(nnodes, max_neigh, bonds, device, steps=None):
     """Is the pair form of the fused step used for a model of this size?
-    ``bonds`` counts the directed bonds."""
+    ``bonds`` counts the directed bonds, ``steps`` the run's steps where they
+    are known."""
     return ((max_neigh > NARROW or bonds >= MIN_BONDS)
+            and _repays(bonds, steps)
             and fits(nnodes, max_neigh, bonds, device))
+
+
+def _repays(bonds, steps):
+    """Do the steps of a run repay the list, which takes 0.1 ms (more, with many
+    bonds) to build?  Calls on one kernel and on pairs break even at 50 steps of
+    37,000 bonds, 27 of 167,000, 7 of 418,000, 4 to 6 of a million, 5 of 3.6
+    million and 2 of 10.6 million; calls of one step take 0.79 against 0.89 ms
+    (37,000 bonds), 1.01 against 1.12 (418,000) and 4.72 against 4.94 (10.6
+    million)."""
+    return steps is None or steps >= 2 + 6_000_000 / (bonds + 80_000)
+
+
+def cy_worthwhile(nnodes, width, bonds, device, steps=None):
+    """The same for PeriPy's CPU integrator, whose calls break even at 7 steps
+    of 37,000 bonds and between 2 and 3 of 167,000; with 891,000 one step is
+    faster on pairs (1.50 against 1.61 ms)."""
+    return ((steps is None or steps * bonds >= 300_000)
+            and fits(nnodes, width, bonds, device))
 
 
 def fits(nnodes, max_neigh, bonds, device):

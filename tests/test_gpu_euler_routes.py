@@ -18,7 +18,8 @@ pytestmark = [pytest.mark.gpu,
 def _run(monkeypatch, setup, route, steps, change):
     import probabilistic_peridynamics_gb300 as pp
     from probabilistic_peridynamics_gb300 import integrators
-    monkeypatch.setattr(integrators, "fits", lambda *_: route == "pairs")
+    monkeypatch.setattr(integrators, "cy_worthwhile",
+                        lambda *_: route == "pairs")
     n = setup["coords"].shape[0]
     integ = pp.Euler(0.5, fused=route != "functions")
     integ.build(n, 3, setup["nlist"].shape[1], setup["coords"],
