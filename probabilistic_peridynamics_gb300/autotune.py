@@ -141,13 +141,11 @@ def _key(integ):
             integ.compensated, integ._may_tile)
 
 
-def wants_tiling(integ):
-    """Does an integrator that may be tiled need its tiling: to time it, or
-    because it is known to be the choice for its planned run?"""
-    if not integ.autotune or _key(integ) not in _cache:
-        return True
-    return choose(*_cache[_key(integ)],
-                  integ.planned_steps).startswith("tiled/")
+def known_choice(integ):
+    """What :func:`choose` takes for the integrator's planned run, or None where
+    its step has not been timed."""
+    timed = _cache.get(_key(integ)) if integ.autotune else None
+    return None if timed is None else choose(*timed, integ.planned_steps)
 
 
 def _apply(integ, choice):
@@ -168,13 +166,14 @@ def _time_setup(integ):
     return 1e3 * (time.perf_counter() - start)
 
 
-def tune_mixed(integ, warmup=3, reps=10):
+def tune_mixed(integ, choice=None, warmup=3, reps=10):
     """Pick the layout and tile shape of a mixed-precision integrator.
 
     Times every tile shape of the untiled kernel and, when the integrator
     was set up tiled, of the tiled kernel, and keeps the one :func:`choose`
-    takes for the integrator's planned run: an integrator whose untiled
-    kernel wins drops its tiling.
+    takes for the integrator's planned run (``choice``, where
+    :func:`known_choice` knows it already): an integrator whose untiled
+    kernel wins drops its tiling.  Called on the context's stream.
 
     :returns: dict ``"layout/variant"`` -> milliseconds per step.
     """
@@ -182,16 +181,15 @@ def tune_mixed(integ, warmup=3, reps=10):
     key = _key(integ)
     if key not in _cache:
         tiled = integ.tiling is not None
-        with integ.context.on_stream():
-            results, setup_ms = {}, 0.0
-            if tiled:
-                results.update(_time_layout(integ, True, warmup, reps))
-            results.update(_time_layout(integ, False, warmup, reps))
-            if tiled:
-                setup_ms = _time_setup(integ)
+        results, setup_ms = {}, 0.0
+        if tiled:
+            results.update(_time_layout(integ, True, warmup, reps))
+        results.update(_time_layout(integ, False, warmup, reps))
+        if tiled:
+            setup_ms = _time_setup(integ)
         _cache[key] = (results, setup_ms)
         torch.cuda.empty_cache()
-    results, setup_ms = _cache[key]
-    with integ.context.on_stream():
-        _apply(integ, choose(results, setup_ms, integ.planned_steps))
-    return results
+    if choice is None:
+        choice = choose(*_cache[key], integ.planned_steps)
+    _apply(integ, choice)
+    return _cache[key][0]

@@ -35,6 +35,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import check, lib
+from .autotune import known_choice, tune_mixed
 from .pairs import CyPairs, DevicePairs, cy_worthwhile, worthwhile
 
 
@@ -449,9 +450,11 @@ class _CUDAIntegrator(Integrator):
         self.damage_d = self._zeros((n,), torch.float64)
         self._parity = 0
         if self.precision == "mixed":
-            from .autotune import tune_mixed, wants_tiling
-            self.tiled = self._may_tile and wants_tiling(self)
-            self.tiling = None
+            choice = known_choice(self)
+            self.tiled = self._may_tile and (choice is None or
+                                             choice.startswith("tiled/"))
+            if not self.tiled:
+                self.tiling = None
             self._create_mixed_buffers()
         self.bond_length_d = None
         self._pairs = None
@@ -486,7 +489,7 @@ class _CUDAIntegrator(Integrator):
             check(lib().pp_mixed_pack(ctypes.byref(self._fargs), 0,
                                       self._stream), "pp_mixed_pack")
             if self.autotune:
-                self.tuning = tune_mixed(self)
+                self.tuning = tune_mixed(self, choice)
         self.planned_steps = None
         self._create_special_buffers()
 

@@ -25,19 +25,19 @@ def test_choice(results, steps, expected):
     assert autotune.choose(results, 5.0, steps) == expected
 
 
-def test_no_tiling_where_it_is_known_not_to_be_taken(monkeypatch):
+def test_choice_that_is_known(monkeypatch):
     integ = types.SimpleNamespace(
         nnodes=10, max_neighbours=8, _kind=1, stiffness_corrections_d=None,
         bond_types_d=None, node_instance_d=None, compensated=False,
         _may_tile=True, autotune=True, planned_steps=200)
     monkeypatch.setattr(autotune, "_cache", {})
-    assert autotune.wants_tiling(integ)  # to time it
+    assert autotune.known_choice(integ) is None  # to be timed
     autotune._cache[autotune._key(integ)] = (TIE, 5.0)
-    assert not autotune.wants_tiling(integ)
+    assert autotune.known_choice(integ) == "untiled/0"
     integ.planned_steps = 20_000
-    assert autotune.wants_tiling(integ)
+    assert autotune.known_choice(integ) == "tiled/0"
     integ.planned_steps, integ.autotune = 200, False
-    assert autotune.wants_tiling(integ)  # as its caller asked
+    assert autotune.known_choice(integ) is None  # as its caller asked
 
 
 def test_simulate_says_how_long_its_run_is(mesh):  # noqa: F811
