@@ -261,7 +261,7 @@ typedef struct pp_fused_args {
     int32_t nregimes;
     int32_t nbond_types;
     int32_t flags;                 /* PP_FLAG_* bits; others must be 0     */
-    int32_t nodes_per_block;       /* PP_FLOAT64: warps per block, 1..8 (0 = 8) */
+    int32_t nodes_per_block;       /* PP_FLOAT64: warps per block, 1..8 (0 = 4) */
     int32_t variant;               /* PP_MIXED tile shape, 0..PP_MIXED_VARIANTS-1:
                                       0: 4 warps x 64 nodes per CTA,
                                       register budget for 8 resident CTAs
@@ -383,7 +383,7 @@ typedef struct pp_pairs {
 int pp_pair_count(const pp_fused_args* args, int32_t* slot_pair, int32_t* row_start,
                   int32_t* scratch, void* stream);
 
-/* Fills pairs->slots, slot_pair (as pp_pair_count left it) and length.
+/* Fills pairs->slots, slot_pair (as pp_pair_count left it), length and vector.
  * *differ (a device word) becomes 1 when the two directions of some bond
  * have other volumes or stiffness corrections. */
 int pp_pair_fill(const pp_fused_args* args, const pp_pairs* pairs, const int32_t* row_start,

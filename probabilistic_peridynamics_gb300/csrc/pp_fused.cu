@@ -20,8 +20,9 @@ namespace pp {
 namespace {
 
 // Four warps a block: 24 warps per SM at 80 registers, and a block's node
-// updates wait for four warps only (measured with more work on the FP64 pipe:
-// 2,000 nodes 19.8 against 20.6 us with eight).
+// updates wait for four warps only (us a step with 2, 4 and 8: 900 nodes in rows
+// of 32 slots 5.1, 5.3, 5.4; 2,116 nodes 6.40, 6.45, 6.58; 7,200 nodes, where
+// pairs take 9.9, 14.8, 13.8, 13.6; 2,000 nodes in rows of 128 14.3, 14.7, 16.3).
 constexpr int kDefaultWarps = 4;
 
 // One warp per node for the bond phase; the node updates of the block's

@@ -12,8 +12,8 @@
 //  k_pair_nodes  one warp per node: the records of its slots summed in the
 //                work-group tree order (pp_common.cuh), then the node update.
 //
-// Both kernels are bound by the binary64 pipe (88 and 85 % busy on the plate of
-// 400,000 nodes in rows of 128 slots: 0.63 + 0.34 ms), so halving the bond
+// Both kernels are bound by the binary64 pipe (88 and 92 % busy on the plate of
+// 400,000 nodes in rows of 128 slots: 0.62 + 0.32 ms), so halving the bond
 // work (1.95 ms in one kernel) outweighs writing and gathering the records (32 bytes
 // a pair written, 32 gathered per slot).  What that pipe does not have to do is
 // kept off it: roots and quotients (pp_exact64.cuh), the reference vectors

@@ -33,7 +33,8 @@ __device__ __forceinline__ d3 load_record_if(const double* p, bool live) {
 
 // The record at p as slot `sp` sees it: negated for a pair's second slot, +0
 // for sp = -1.  By bits: a selected negation is an instruction of the
-// binary64 pipe.
+// binary64 pipe.  (A component that is zero gets the other sign of zero than the
+// slot's own product has: equal as a number, and so are the sums.)
 __device__ __forceinline__ d3 signed_record(const double* p, int sp) {
     const d3 v = load_record_if(p, sp != -1);
     const long long flip = sp < -1 ? (long long)0x8000000000000000ull : 0;
