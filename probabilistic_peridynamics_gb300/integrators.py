@@ -213,6 +213,10 @@ class _CUDAIntegrator(Integrator):
     _kind = None          # PP_EULER / PP_EULER_CROMER / PP_VELOCITY_VERLET
     _dynamic = False      # needs densities, ud, udd
 
+    #: Steps of the run that the next create_buffers begins, where its caller
+    #: knows them (Model.simulate does).
+    planned_steps = None
+
     def __init__(self, dt, context=None, fused=True, precision="float64",
                  compensated=False, nodes_per_block=0, use_graph=True,
                  autotune=True, tiled=True):
@@ -237,9 +241,6 @@ class _CUDAIntegrator(Integrator):
         self._may_tile = bool(tiled) and precision == "mixed"
         self.tiled = self._may_tile  # the layout of the current buffers
         self.tiling = None
-        # steps of the run that the next create_buffers begins, where its
-        # caller knows them (Model.simulate does)
-        self.planned_steps = None
         self.tile_target = 125  # nodes per brick of the internal order
         self._order = None
         self.tuning = None
@@ -837,6 +838,10 @@ class Euler(Integrator):
     :meth:`create_buffers` raises ValueError otherwise.
     """
 
+    #: Steps of the run that the next create_buffers begins, where its caller
+    #: knows them (Model.simulate does).
+    planned_steps = None
+
     def __init__(self, dt, device_context=None, fused=True):
         """Create an :class:`Euler` integrator object.
 
@@ -854,9 +859,6 @@ class Euler(Integrator):
         self.fused = bool(fused)
         # Not a device-layout integrator: Model builds the compact layout
         self.context = None
-        # steps of the run that the next create_buffers begins, where its
-        # caller knows them (Model.simulate does)
-        self.planned_steps = None
         self._device = device_context
         lib()  # fail loudly now if the CUDA library is missing
 
